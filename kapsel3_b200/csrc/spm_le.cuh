@@ -369,6 +369,33 @@ __global__ void r_le_reset(Grid g, const T *__restrict__ u0, const T *__restrict
     }
 }
 
+// Block-wide sum of K doubles (blockDim.x a multiple of 32, <= 1024); the
+// result is valid in thread 0.
+template <int K>
+__device__ __forceinline__ void block_sumK(double v[K]) {
+    __shared__ double red[32][K];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < K; k++)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    __syncthreads();
+    if (lane == 0)
+#pragma unroll
+        for (int k = 0; k < K; k++) red[wid][k] = v[k];
+    __syncthreads();
+    if (wid == 0) {
+        const int nw = blockDim.x >> 5;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            double a = lane < nw ? red[lane][k] : 0.0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            v[k] = a;
+        }
+    }
+}
+
 // Field reductions of the step: Calc_shear_rate_eff's average gradient of the
 // oblique x velocity (sp_3d_ns.h:166-203) and the Reynolds stress of the
 // Cartesian velocity (fluid_solver.h:165-183).  One block-level partial per
@@ -409,18 +436,27 @@ __global__ void r_le_reductions(Grid g, const T *__restrict__ u0, const T *__res
     }
 }
 
+// The sums over CTA partials and over particles are one block's: each thread
+// adds every kLeFinishThreads-th term, a tree over the block follows, so the
+// order is fixed.  One thread walking the list waits for every load in turn
+// (2368 partials: 86 us a launch on B200, 128^3 and 64^3 alike; a block of
+// 1024 takes 3 us).
+constexpr int kLeFinishThreads = 1024;
+
 // which = 0: Shear_rate_eff = shear_rate + ivol * sum (set once per step)
 // which = 1: Inertia_stress = -ivol * RHO * sum
-__global__ void k_le_finish_reduction(LEDev *le, const double *partial, int nparts, int which, double ivol,
-                                      double rho, double shear_rate) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0;
-    for (int i = 0; i < nparts; i++) s += partial[i];
+__global__ void __launch_bounds__(kLeFinishThreads)
+    k_le_finish_reduction(LEDev *le, const double *__restrict__ partial, int nparts, int which, double ivol, double rho,
+                          double shear_rate) {
+    double s[1] = {0.0};
+    for (int i = threadIdx.x; i < nparts; i += kLeFinishThreads) s[0] += partial[i];
+    block_sumK<1>(s);
+    if (threadIdx.x != 0) return;
     if (which == 0) {
-        le->correction = s * ivol;
+        le->correction = s[0] * ivol;
         le->srate_eff  = shear_rate + le->correction;
     } else {
-        le->reynolds = -ivol * rho * s;
+        le->reynolds = -ivol * rho * s[0];
     }
 }
 
@@ -531,33 +567,6 @@ __global__ void s_le_up_scatter(Grid g, Phys ph, const double *__restrict__ x, c
     atomicAdd(&up2[s.idx], (T)(vs[2] * wgt));
 }
 
-// Block-wide sum of K doubles (blockDim.x a multiple of 32, <= 1024); the
-// result is valid in thread 0.
-template <int K>
-__device__ __forceinline__ void block_sumK(double v[K]) {
-    __shared__ double red[32][K];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < K; k++)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-    __syncthreads();
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < K; k++) red[wid][k] = v[k];
-    __syncthreads();
-    if (wid == 0) {
-        const int nw = blockDim.x >> 5;
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            double a = lane < nw ? red[lane][k] : 0.0;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-            v[k] = a;
-        }
-    }
-}
-
 // Calc_f_hydro_correct_precision_OBL (md_force.cxx:508-745): force and torque
 // of each particle, and per-particle partial sums of the Hydro_force and
 // Hydro_force_new fields' totals (all that Mean_shear_stress reads of them).
@@ -651,25 +660,23 @@ __global__ void s_le_hydro_force(Grid g, Phys ph, const double *__restrict__ x, 
 
 // Totals of the hydrodynamic stress fields and the LJ stress
 // (Calc_hydro_stress, fluid_solver.h:253-279; Force_OBL, particle_solver.h:113-128).
-__global__ void k_le_stress_finish(LEDev *le, const double *ppart, const double *lj_stress, int np, double ivol,
-                                   double ivolume_lj, double dt, double rho) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double A = 0, Y = 0, F = 0, V = 0, Nw = 0, M = 0, L = 0;
-    for (int p = 0; p < np; p++) {
-        const double *pp = ppart + kLePart * p;
-        A += pp[0];
-        Y += pp[1];
-        F += pp[2];
-        V += pp[3];
-        Nw += pp[4];
-        M += pp[5];
-        L += lj_stress[p];
+__global__ void __launch_bounds__(kLeFinishThreads)
+    k_le_stress_finish(LEDev *le, const double *__restrict__ ppart, const double *__restrict__ lj_stress, int np,
+                       double ivol, double ivolume_lj, double dt, double rho) {
+    double t[7] = {0, 0, 0, 0, 0, 0, 0};  // A, Y, force, volume, new, mdf, LJ
+    for (int p = threadIdx.x; p < np; p += kLeFinishThreads) {
+        const double *pp = ppart + (size_t)kLePart * p;
+#pragma unroll
+        for (int k = 0; k < 6; k++) t[k] += pp[k];
+        t[6] += lj_stress[p];
     }
-    const double sum_volume = V / rho;
-    const double hf_old     = A - M - (F / sum_volume) * Y;
+    block_sumK<7>(t);
+    if (threadIdx.x != 0) return;
+    const double sum_volume = t[3] / rho;
+    const double hf_old     = t[0] - t[5] - (t[2] / sum_volume) * t[1];
     le->hydro_old           = -hf_old * ivol / dt;
-    le->hydro_new           = -Nw * ivol / dt;
-    le->lj                  = L * ivolume_lj;
+    le->hydro_new           = -t[4] * ivol / dt;
+    le->lj                  = t[6] * ivolume_lj;
 }
 
 // PBC_OBL wrap after the position update (particle_solver.cxx:283-334,
