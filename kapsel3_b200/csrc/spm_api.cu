@@ -28,6 +28,7 @@
 #include "spm_electrolyte.cuh"
 #include "spm_janus.cuh"
 #include "spm_sns.cuh"
+#include "spm_xfuse.cuh"
 
 using namespace spm;
 
@@ -730,35 +731,72 @@ double stencil_bytes(const spm_ctx *c, int kind) {
 // run, FFT stages to L, which is either the run itself or a pool lead whose
 // FFT launches cover the same slots of every run of the pool.
 // ---------------------------------------------------------------------------
-// u (real space) from zeta.  truncate = 1 is the step's Zeta_k2u (2/3 rule
-// applied, pruned passes); truncate = 0 keeps every mode (state getters).
+// One fused X pass over slots `slot`.. of every run of L (spm_xfuse.cuh).
+// Returns false where it does not apply; the caller then launches the separate
+// X pass and k-space kernel.  Algorithmic bytes: the transformed fields' x
+// lines read and written plus zeta (and its compensation) read and written.
+template <typename T, int OP, bool INV>
+int x_fused_pass(spm_ctx *L, int slot, int ts_inc, bool &done) {
+    done = false;
+    if (!L->use_tma) return SPM_OK;
+    const Grid &g = L->g;
+    XArgs<T>    A{};
+    A.g = g;
+    A.z0 = L->cx<T>(Z0), A.z1 = L->cx<T>(Z1);
+    A.zl0 = OP == kXZeta ? nullptr : L->zl<T>(0), A.zl1 = OP == kXZeta ? nullptr : L->zl<T>(1);
+    A.u  = L->cx<T>(slot);
+    A.rw = L->rw;
+    A.run_stride = L->fstride_c, A.slot_stride = L->slot_stride_c;
+    A.ts_inc = ts_inc;
+    A.nu = L->ph.nu, A.dt = L->ph.dt;
+    const int    nf   = OP == kXNs ? 5 : OP == kXProj ? 3 : 0;
+    const double cols = (double)outer_count(g.ny, g.trn[1]) * g.trn[2] * L->fft_runs * sizeof(cplx<T>);
+    const double box  = box_bytes<T>(L, OP == kXZeta ? 2 : A.zl0 ? 8 : 4);
+    cudaEvent_t  pa   = prof_mark(L);
+    const cudaError_t e = x_fused<T, OP, INV>(plan_of<T>(L), A, L->fft_runs, L->nslots - slot, L->st);
+    if (e == cudaErrorNotSupported) return SPM_OK;
+    SPM_CUDA_CHECK(e);
+    prof_done(L, pa, OP == kXZeta ? "x_zeta_u" : OP == kXNs ? "x_ns_update" : "x_project",
+              (nf + (INV ? 3 : 0)) * cols * g.nx + box);
+    L->launches++;
+    done = true;
+    return SPM_OK;
+}
+
+// u of the truncated zeta up to its inverse X pass, in U0..U2 (real in x).
 template <typename T>
-int zeta_to_velocity(spm_ctx *L, int truncate, bool have_u_hat = false) {
+int zeta_to_ux(spm_ctx *L) {
+    bool done;
+    SPM_TRY((x_fused_pass<T, kXZeta, true>(L, U0, 0, done)));
+    if (done) return SPM_OK;
+    PLAUNCH(L, "k_zeta_to_u", box_bytes<T>(L, 5), (k_zeta_to_u<T, 1>), L->box_grid(), 256, 0, L->g, L->cx<T>(Z0),
+            L->cx<T>(Z1), L->uk_dc, L->cx<T>(U0), L->cx<T>(U1), L->cx<T>(U2), 1, L->fstride_c);
+    return fft_strided_pass<T, +1>(L, U0, 3, 0, prune_inverse(L->g, 0));
+}
+
+// u (real space) from zeta.  truncate = 1 is the step's Zeta_k2u (2/3 rule
+// applied, pruned passes; have_ux: U0..U2 already hold it up to the inverse X
+// pass); truncate = 0 keeps every mode (state getters).
+template <typename T>
+int zeta_to_velocity(spm_ctx *L, int truncate, bool have_ux = false) {
     if (!truncate) {
         LAUNCH(L, (k_zeta_to_u<T, 0>), L->pw_grid(), 256, 0, L->g, L->cx<T>(Z0), L->cx<T>(Z1), L->uk_dc, L->cx<T>(U0),
                L->cx<T>(U1), L->cx<T>(U2), 0, L->fstride_c);
         return fft_inv_packed<T>(L, U0, 3);
     }
-    int rc;
-    if (!have_u_hat)
-        PLAUNCH(L, "k_zeta_to_u", box_bytes<T>(L, 5), (k_zeta_to_u<T, 1>), L->box_grid(), 256, 0, L->g,
-                L->cx<T>(Z0), L->cx<T>(Z1), L->uk_dc, L->cx<T>(U0), L->cx<T>(U1), L->cx<T>(U2), 1, L->fstride_c);
-    if ((rc = fft_strided_pass<T, +1>(L, U0, 3, 0, prune_inverse(L->g, 0))) != SPM_OK) return rc;
-    if ((rc = fft_strided_pass<T, +1>(L, U0, 3, 1, prune_inverse(L->g, 1))) != SPM_OK) return rc;
+    if (!have_ux) SPM_TRY(zeta_to_ux<T>(L));
+    SPM_TRY((fft_strided_pass<T, +1>(L, U0, 3, 1, prune_inverse(L->g, 1))));
     return z_pass<T>(L, U0, 3, false, L->g.trn[2]);
 }
 
-// NS_solver_slavedEuler (fluid_solver.cxx:348-374).  with_u: the update also
-// writes the velocity of the new zeta (the k_zeta_to_u that Zeta_k2u of the
-// step would run next) into U0..U2, k = 0 with FIX_CELL applied.
+// NS_solver_slavedEuler (fluid_solver.cxx:348-374).  with_u: followed by
+// FIX_CELLxyz on `nr` runs and the velocity of the new zeta up to its inverse
+// X pass (zeta_to_velocity's have_ux).
 template <typename T>
-int ns_solver(spm_ctx *L, bool with_u = false) {
-    int rc;
+int ns_solver(spm_ctx *L, int nr = 1, bool with_u = false) {
     // zeta -> u_hat (truncated) -> inverse x, y passes
-    PLAUNCH(L, "k_zeta_to_u", box_bytes<T>(L, 5), (k_zeta_to_u<T, 1>), L->box_grid(), 256, 0, L->g, L->cx<T>(Z0),
-            L->cx<T>(Z1), L->uk_dc, L->cx<T>(U0), L->cx<T>(U1), L->cx<T>(U2), 1, L->fstride_c);
-    if ((rc = fft_strided_pass<T, +1>(L, U0, 3, 0, prune_inverse(L->g, 0))) != SPM_OK) return rc;
-    if ((rc = fft_strided_pass<T, +1>(L, U0, 3, 1, prune_inverse(L->g, 1))) != SPM_OK) return rc;
+    SPM_TRY(zeta_to_ux<T>(L));
+    SPM_TRY((fft_strided_pass<T, +1>(L, U0, 3, 1, prune_inverse(L->g, 1))));
     // inverse z + products + forward z in one pass, then forward y, x passes
     {
         const double rows = (double)L->fft_runs * L->g.nx * L->g.ny;
@@ -768,13 +806,25 @@ int ns_solver(spm_ctx *L, bool with_u = false) {
         prof_done(L, pa, "z_products", rows * (3.0 * L->g.trn[2] + 5.0 * L->g.kz_span()) * sizeof(cplx<T>));
     }
     L->launches++;
-    if ((rc = fft_strided_pass<T, -1>(L, U0, 5, 1, prune_forward(L->g, 1))) != SPM_OK) return rc;
-    if ((rc = fft_strided_pass<T, -1>(L, U0, 5, 0, prune_forward(L->g, 0))) != SPM_OK) return rc;
-    PLAUNCH(L, "k_ns_update", box_bytes<T>(L, (L->compensated() ? 13 : 9) + (with_u ? 3 : 0)), (k_ns_update<T, 2>),
+    SPM_TRY((fft_strided_pass<T, -1>(L, U0, 5, 1, prune_forward(L->g, 1))));
+    bool done;
+    if (with_u)
+        SPM_TRY((x_fused_pass<T, kXNs, true>(L, U0, 0, done)));
+    else
+        SPM_TRY((x_fused_pass<T, kXNs, false>(L, U0, 0, done)));
+    if (done) return SPM_OK;
+    SPM_TRY((fft_strided_pass<T, -1>(L, U0, 5, 0, prune_forward(L->g, 0))));
+    // FP64: the update writes u_hat of the new zeta as well, one k_zeta_to_u
+    // fewer.  Measured on B200 at 256^3 the fused update took 82 us against 60 +
+    // 37 us; in FP32 it took 73 us against 44 + 25 us, so FP32 keeps two kernels.
+    const bool u_too = with_u && L->fp64();
+    PLAUNCH(L, "k_ns_update", box_bytes<T>(L, (L->compensated() ? 13 : 9) + (u_too ? 3 : 0)), (k_ns_update<T, 2>),
             L->box_grid(), 256, 0, L->g, L->cx<T>(Z0), L->cx<T>(Z1), L->cx<T>(U0), L->cx<T>(U1), L->cx<T>(U2),
             L->cx<T>(A0), L->cx<T>(A1), L->ph.nu, L->ph.dt, L->fstride_c, L->zl<T>(0), L->zl<T>(1),
-            with_u ? L->rw : (const RunWords *)nullptr);
-    return SPM_OK;
+            u_too ? L->rw : (const RunWords *)nullptr);
+    if (!with_u) return SPM_OK;
+    LAUNCH(L, k_fix_cell, (nr + 127) / 128, 128, 0, L->rw, nr);
+    return u_too ? fft_strided_pass<T, +1>(L, U0, 3, 0, prune_inverse(L->g, 0)) : zeta_to_ux<T>(L);
 }
 
 // Shared-profile scatters (Make_phi_particle_sum, make_phi.cxx:226-247;
@@ -918,17 +968,21 @@ int clear_scatter_slots(spm_ctx *L) {
 
 // Rigidity projection of the step: the forward transform of f (scattered by
 // s_f_scatter_cached, or up itself when u = 0 at initialisation), then the
-// projection and the update of zeta and uk_dc closed in k space
-// (k_project_add_curl).
+// projection and the update of zeta and uk_dc closed in k space, and the step
+// counters of `nr` runs advanced by ts_inc.
 template <typename T>
-int rigidity_projection(spm_ctx *L) {
+int rigidity_projection(spm_ctx *L, int nr, int ts_inc) {
     int rc;
     if ((rc = z_pass<T>(L, UP0, 3, true, 1 << 30, L->g.kz_span())) != SPM_OK) return rc;
     if ((rc = fft_strided_pass<T, -1>(L, UP0, 3, 1, prune_forward(L->g, 1))) != SPM_OK) return rc;
+    bool done;
+    SPM_TRY((x_fused_pass<T, kXProj, false>(L, UP0, ts_inc, done)));
+    if (done) return SPM_OK;
     if ((rc = fft_strided_pass<T, -1>(L, UP0, 3, 0, prune_forward(L->g, 0))) != SPM_OK) return rc;
     PLAUNCH(L, "k_project_add_curl", box_bytes<T>(L, L->compensated() ? 11 : 7), (k_project_add_curl<T, 2>),
             L->box_grid(), 256, 0, L->g, L->cx<T>(UP0), L->cx<T>(UP1), L->cx<T>(UP2), L->cx<T>(Z0), L->cx<T>(Z1),
             L->uk_dc, L->fstride_c, L->zl<T>(0), L->zl<T>(1));
+    if (ts_inc) LAUNCH(L, k_ts_advance, (nr + 127) / 128, 128, 0, L->rw, nr);
     return SPM_OK;
 }
 
@@ -1017,15 +1071,15 @@ int step_ns_runs(spm_ctx *L, spm_ctx *const *R, int nr) {
         if (rc != SPM_OK) return rc;
     }
     if (L->overlap) SPM_CUDA_CHECK(cudaEventRecord(L->ev_join, side));
-    // FP64: the update writes u_hat of the new zeta as well (unless the shear
-    // sustaining step changes zeta in between), one k_zeta_to_u fewer.  Measured
-    // on B200 at 256^3 the fused update took 82 us against 60 + 37 us; in FP32 it
-    // took 73 us against 44 + 25 us, so FP32 keeps the two kernels.
-    const bool fuse_u = L->P.equation != SPM_EQ_SHEAR_NAVIER_STOKES && L->fp64();
-    if ((rc = ns_solver<T>(L, fuse_u)) != SPM_OK) return rc;
-    if (L->P.equation == SPM_EQ_SHEAR_NAVIER_STOKES) SPM_TRY(shear_sustain<T>(L));  // lone runs only
-    LAUNCH(L, k_fix_cell, (nr + 127) / 128, 128, 0, L->rw, nr);
-    if ((rc = zeta_to_velocity<T>(L, 1, fuse_u)) != SPM_OK) return rc;
+    if (L->P.equation == SPM_EQ_SHEAR_NAVIER_STOKES) {  // lone runs only
+        SPM_TRY(ns_solver<T>(L));
+        SPM_TRY(shear_sustain<T>(L));
+        LAUNCH(L, k_fix_cell, (nr + 127) / 128, 128, 0, L->rw, nr);
+        SPM_TRY(zeta_to_velocity<T>(L, 1));
+    } else {
+        SPM_TRY(ns_solver<T>(L, nr, true));
+        SPM_TRY(zeta_to_velocity<T>(L, 1, true));
+    }
     if (L->overlap) SPM_CUDA_CHECK(cudaStreamWaitEvent(L->st, L->ev_join, 0));  // join
     for (int r = 0; r < nr; r++) {
         spm_ctx *c = R[r];
@@ -1053,9 +1107,8 @@ int step_ns_runs(spm_ctx *L, spm_ctx *const *R, int nr) {
                 c->real<T>(U0), c->real<T>(U1), c->real<T>(U2), c->real<T>(UP0), c->real<T>(UP1), c->real<T>(UP2));
     }
     if (L->sns) SPM_TRY(shear_diagnostics<T>(L));  // lone Shear_Navier_Stokes runs
-    if ((rc = rigidity_projection<T>(L)) != SPM_OK) return rc;
+    if ((rc = rigidity_projection<T>(L, nr, 1)) != SPM_OK) return rc;
     if (L->sns && L->P.shear_ac) SPM_TRY(shear_inertia<T>(L));
-    LAUNCH(L, k_ts_advance, (nr + 127) / 128, 128, 0, L->rw, nr);
     for (int r = 0; r < nr; r++) {
         R[r]->ts++;
         R[r]->time += R[r]->ph.dt;
@@ -1077,7 +1130,7 @@ int initialize_impl(spm_ctx *c) {
     if ((rc = up_scatter<T>(c)) != SPM_OK) return rc;
     // u = Zeta_k2u(zeta = 0) = 0
     if ((rc = zeta_to_velocity<T>(c, 1)) != SPM_OK) return rc;
-    if ((rc = rigidity_projection<T>(c)) != SPM_OK) return rc;
+    if ((rc = rigidity_projection<T>(c, 1, 0)) != SPM_OK) return rc;
     LAUNCH(c, k_zero3, 1, 32, 0, c->uk_dc);
     if (c->sns) SPM_CUDA_CHECK(cudaMemsetAsync(c->sns, 0, kSnsWords * sizeof(double), c->st));
     // shear runs start with v_x = omega_z = 0 (init_particle.cxx:768-781)

@@ -171,7 +171,7 @@ struct FFTPlan {
         auto        make = [&](CUtensorMap *m, int lines) {
             const uint32_t box[4] = {(uint32_t)(2 * W_T), axis == 1 ? (uint32_t)lines : 1u,
                                      axis == 1 ? 1u : (uint32_t)lines, 1u};
-            return make_map_4d<T>(m, data, dims, strides, box);
+            return make_map<T>(m, data, dims, strides, box);
         };
         if (!make(&lmap, pruned_box_lines(n, pr.line_trn)) || !make(&smap, pruned_box_lines(n, pr.out_trn)))
             return cudaErrorNotSupported;

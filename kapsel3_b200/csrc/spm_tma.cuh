@@ -43,18 +43,22 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
 // err is given).
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, unsigned int *err,
                                           unsigned long long limit_ns) {
-    const unsigned           a  = smem_addr(bar);
-    const unsigned long long t0 = global_ns();
-    for (;;) {
-        unsigned done;
+    const unsigned a    = smem_addr(bar);
+    auto           done = [&] {
+        unsigned d;
         asm volatile(
             "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
+            : "=r"(d)
             : "r"(a), "r"(parity)
             : "memory");
-        if (done) return true;
-        if (global_ns() - t0 > limit_ns) break;
-    }
+        return d != 0;
+    };
+    // a phase that is complete already costs no read of the global timer
+    if (done()) return true;
+    const unsigned long long t0 = global_ns();
+    do {
+        if (done()) return true;
+    } while (global_ns() - t0 <= limit_ns);
     if (err) atomicOr(err, SPM_DEVERR_TIMEOUT);
     return false;
 }
@@ -66,6 +70,16 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, i
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
         "%5}], [%6];" ::"r"(smem_addr(dst)),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_addr(bar))
+        : "memory");
+}
+
+// 5D tiled TMA load global -> shared, completion counted on `bar`.
+__device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4,
+                                            uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
+        "%5, %6}], [%7];" ::"r"(smem_addr(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_addr(bar))
         : "memory");
 }
 
@@ -113,16 +127,17 @@ inline EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// 4D map over a field array of element type T (float/double), dims given
-// innermost first in elements, strides (dims 1..3) in bytes.
-template <typename T>
-inline bool make_map_4d(CUtensorMap *map, void *base, const uint64_t dims[4], const uint64_t strides_bytes[3],
-                        const uint32_t box[4]) {
+// R-dimensional map over a field array of element type T (float/double),
+// dims given innermost first in elements, strides (dims 1..R-1) in bytes.
+template <typename T, int R>
+inline bool make_map(CUtensorMap *map, void *base, const uint64_t (&dims)[R], const uint64_t (&strides_bytes)[R - 1],
+                     const uint32_t (&box)[R]) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    cuuint32_t estr[R];
+    for (int i = 0; i < R; i++) estr[i] = 1;
     const CUtensorMapDataType dt = sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    const CUresult r = fn(map, dt, 4, base, reinterpret_cast<const cuuint64_t *>(dims),
+    const CUresult r = fn(map, dt, R, base, reinterpret_cast<const cuuint64_t *>(dims),
                           reinterpret_cast<const cuuint64_t *>(strides_bytes), reinterpret_cast<const cuuint32_t *>(box),
                           estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
