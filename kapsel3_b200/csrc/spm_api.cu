@@ -96,7 +96,8 @@ cudaError_t dev_pool(DevMem &m, int dev, DevMemPool **out) {
     return cudaSuccess;
 }
 
-cudaError_t dev_alloc(void **p, size_t bytes) {
+}  // namespace
+cudaError_t spm::dev_alloc(void **p, size_t bytes) {
     for (int n = g_fail_allocs.load(); n > 0; n = g_fail_allocs.load())
         if (g_fail_allocs.compare_exchange_weak(n, n - 1)) {
             *p = nullptr;
@@ -114,7 +115,7 @@ cudaError_t dev_alloc(void **p, size_t bytes) {
     m.live[*p] = dev;
     return cudaSuccess;
 }
-void dev_free(void *p) {
+void spm::dev_free(void *p) {
     if (!p) return;
     DevMem                     &m = dev_mem();
     std::lock_guard<std::mutex> lk(m.mu);
@@ -124,7 +125,6 @@ void dev_free(void *p) {
     if (pit != m.pools.end()) cudaFreeAsync(p, pit->second.st);
     m.live.erase(it);
 }
-}  // namespace
 
 #undef SPM_CUDA_CHECK
 #define SPM_CUDA_CHECK(expr)                                                                             \
@@ -186,6 +186,10 @@ struct spm_ctx {
     FFTPlan<double> *pp64 = &plan64;  // the plans in use (a pool's runs use the lead's)
     FFTPlan<float>  *pp32 = &plan32;
     spm_pool        *pool = nullptr;  // pool this run belongs to (null for a lone run)
+    // a pool lead's runs as their particle kernels see them (PRun<T>[], device),
+    // the largest particle count and stencil among them
+    void            *pruns = nullptr;
+    int              prun_np = 0, prun_cells = 0;
     int *        cells   = nullptr;
     int *        lj_list = nullptr;  // LJ cell list: count[ncell], cell_of[np], bins[ncell][kLjBin]
     int *        sc_idx  = nullptr;  // stencil cache of the NS step: grid index per (particle, cell)
@@ -562,22 +566,20 @@ FFTPlan<float> &plan_of<float>(spm_ctx *c) {
     return *c->pp32;
 }
 
-// Strided (Y/X) FFT pass over `nf` slots of this context: the persistent TMA
-// kernel when it applies, else the direct-load kernel.  A pool lead batches
-// the same slots of all its runs (run-consecutive within a slot) into one
-// launch per slot.
+// Strided (Y/X) FFT pass over `nf` slots of this context, for a pool lead the
+// same slots of all its runs in one launch: the persistent TMA kernel when it
+// applies, else the direct-load kernel (one launch per slot of a pool).
 template <typename T, int DIR>
 cudaError_t strided_dispatch(spm_ctx *c, int slot, int nf, int axis, PassPrune pr) {
-    auto one = [&](cplx<T> *base, int nfields, size_t stride) {
-        if (c->use_tma) {
-            cudaError_t e = plan_of<T>(c).template strided_tma<DIR>(base, nfields, stride, axis, c->st, pr);
-            if (e != cudaErrorNotSupported) return e;
-        }
-        return plan_of<T>(c).template strided<DIR>(base, nfields, stride, axis, c->st, pr);
-    };
-    if (c->fft_runs == 1) return one(c->cx<T>(slot), nf, c->slot_stride_c);
+    if (c->use_tma) {
+        cudaError_t e = plan_of<T>(c).template strided_tma<DIR>(c->cx<T>(slot), nf, c->slot_stride_c, c->fft_runs,
+                                                                c->fstride_c, axis, c->st, pr);
+        if (e != cudaErrorNotSupported) return e;
+    }
+    if (c->fft_runs == 1)
+        return plan_of<T>(c).template strided<DIR>(c->cx<T>(slot), nf, c->slot_stride_c, axis, c->st, pr);
     for (int k = 0; k < nf; k++) {
-        cudaError_t e = one(c->cx<T>(slot + k), c->fft_runs, c->fstride_c);
+        cudaError_t e = plan_of<T>(c).template strided<DIR>(c->cx<T>(slot + k), c->fft_runs, c->fstride_c, axis, c->st, pr);
         if (e != cudaSuccess) return e;
         c->launches += k > 0;
     }
@@ -627,27 +629,18 @@ template <typename T, int DIR>
 int fft_strided_pass(spm_ctx *c, int slot, int nf, int axis) {
     return fft_strided_pass<T, DIR>(c, slot, nf, axis, PassPrune::full(c->g.hnz));
 }
-// z passes over `nf` slots (one launch per slot when batching runs).
+// z passes over `nf` slots of every batched run.
 // kz_keep: inverse inputs kz >= kz_keep read as zero; kz_span: forward
 // outputs kz >= kz_span left unwritten (both: pruned transforms).
 template <typename T>
 int z_pass_launch(spm_ctx *c, int slot, int nf, bool forward, int kz_keep, int kz_span) {
-    const T scale = (T)(1.0 / ((double)c->g.nx * c->g.ny * c->g.nz));
-    auto    one   = [&](int s, int nfields, size_t stride) {
-        return forward ? plan_of<T>(c).z_r2c(c->real<T>(s), c->cx<T>(s), nfields, 2 * stride, stride, c->st,
-                                             kz_span)
-                       : plan_of<T>(c).z_c2r(c->cx<T>(s), c->real<T>(s), nfields, stride, 2 * stride, scale, c->st,
-                                             kz_keep);
-    };
-    if (c->fft_runs == 1) {
-        SPM_CUDA_CHECK(one(slot, nf, c->slot_stride_c));
-        c->launches++;
-        return SPM_OK;
-    }
-    for (int k = 0; k < nf; k++) {
-        SPM_CUDA_CHECK(one(slot + k, c->fft_runs, c->fstride_c));
-        c->launches++;
-    }
+    const T      scale = (T)(1.0 / ((double)c->g.nx * c->g.ny * c->g.nz));
+    const size_t fs    = c->slot_stride_c;
+    SPM_CUDA_CHECK(forward ? plan_of<T>(c).z_r2c(c->real<T>(slot), c->cx<T>(slot), nf, 2 * fs, fs, c->st, kz_span,
+                                                 c->fft_runs, c->fstride_c)
+                           : plan_of<T>(c).z_c2r(c->cx<T>(slot), c->real<T>(slot), nf, fs, 2 * fs, scale, c->st,
+                                                 kz_keep, c->fft_runs, c->fstride_c));
+    c->launches++;
     return SPM_OK;
 }
 template <typename T>
@@ -988,29 +981,51 @@ int rigidity_projection(spm_ctx *L, int nr, int ts_inc) {
 
 int particle_blocks(spm_ctx *c) { return (c->ph.np + 127) / 128; }
 
+// The particle kernels' view of run c (PRun).
+template <typename T>
+PRun<T> prun_of(spm_ctx *c) {
+    PRun<T> R{};
+    R.ph = c->ph, R.ps = c->ps;
+    R.cells = c->cells, R.ncells = c->ncells;
+    R.vel   = !c->rigid() && c->ph.janus_prop != SPM_JANUS_SQUIRMER;
+    // obstacles draw no noise (fluct.cxx:23)
+    R.noise   = c->P.kbt > 0.0 && c->ph.janus_prop != SPM_JANUS_OBSTACLE;
+    R.phi_sum = c->real<T>(PHIS);
+    R.u0 = c->real<T>(U0), R.u1 = c->real<T>(U1), R.u2 = c->real<T>(U2);
+    R.f0 = c->real<T>(UP0), R.f1 = c->real<T>(UP1), R.f2 = c->real<T>(UP2);
+    R.sc_idx = c->sc_idx, R.sc_w = c->sc_w;
+    if (c->lj_list && lj_cell_list_applies(c->ph)) {
+        R.lj_ncell   = lj_ncell(c->ph);
+        R.lj_count   = c->lj_list;
+        R.lj_cell_of = R.lj_count + R.lj_ncell;
+        R.lj_bins    = R.lj_cell_of + c->ph.np;
+    }
+    if (c->rigid()) R.rid = c->rg.rid, R.f_lo = c->rg.f_lo;
+    R.ts = c->ts_dev, R.mt = c->mt, R.err = c->err;
+    return R;
+}
+
 // The LJ forces of Force() (particle_solver.h:88-111) with the constant
 // body force: through the cell list (particles binned per 16-DX cell, one warp
 // per particle over the 27 neighbour cells) when the grid has at least one
 // such cell per axis, as the reference's cell list needs; else the scan over
 // all partners with the reference's pair multiplicity (p_forces).
-int lj_forces(spm_ctx *c, const Phys &ph) {
+int lj_forces(spm_ctx *c, const Phys &ph, bool clear = true) {
     if (ph.np == 0) return SPM_OK;
     if (!c->lj_list || !lj_cell_list_applies(ph)) {
         PLAUNCH(c, "p_forces", 0.0, p_forces, (ph.np + 3) / 4, 128, 0, ph, c->ps, 0, 0.0,
                 c->rigid() ? c->rg.rid : nullptr, c->rigid() ? c->rg.f_lo : nullptr, (const double *)nullptr);
         return SPM_OK;
     }
-    const int ncell   = lj_ncell(ph);
-    int      *count   = c->lj_list;
-    int      *cell_of = count + ncell;
-    int      *bins    = cell_of + ph.np;
+    PRun<double> R = prun_of<double>(c);
+    R.ph           = ph;
     if (ph.lj_on && ph.janus_prop != 3) {
-        SPM_CUDA_CHECK(cudaMemsetAsync(count, 0, (size_t)ncell * sizeof(int), c->st));
-        PLAUNCH(c, "p_cells_bin", 0.0, p_cells_bin, (ph.np + 127) / 128, 128, 0, ph, c->ps.x, count, cell_of, bins,
-                c->err);
+        if (clear) SPM_CUDA_CHECK(cudaMemsetAsync(R.lj_count, 0, (size_t)R.lj_ncell * sizeof(int), c->st));
+        PLAUNCH(c, "p_cells_bin", 0.0, (p_cells_bin<double, false>), (ph.np + 127) / 128, 128, 0, R,
+                (const PRun<double> *)nullptr);
     }
-    PLAUNCH(c, "p_forces_cells", 0.0, p_forces_cells, (ph.np + 3) / 4, 128, 0, ph, c->ps, count, cell_of, bins,
-            c->rigid() ? c->rg.rid : nullptr, c->rigid() ? c->rg.f_lo : nullptr);
+    PLAUNCH(c, "p_forces_cells", 0.0, (p_forces_cells<double, false>), (ph.np + 3) / 4, 128, 0, R,
+            (const PRun<double> *)nullptr);
     return SPM_OK;
 }
 
@@ -1023,6 +1038,41 @@ int truncate_if_dirty(spm_ctx *c) {
     LAUNCH(c, k_truncate2<T>, c->grid_blocks(), 256, 0, c->g, c->cx<T>(Z0), c->cx<T>(Z1));
     if (c->compensated()) LAUNCH(c, k_truncate2<T>, c->grid_blocks(), 256, 0, c->g, c->cx<T>(ZL0), c->cx<T>(ZL1));
     c->zeta_dirty = false;
+    return SPM_OK;
+}
+
+// The particle work of a pool's step, one launch per kernel over all runs
+// (L->pruns, blockIdx.z = run; the grid covers the largest run): what needs
+// only the previous step's state, and what follows the fluid solve.
+template <typename T>
+int pool_side_work(spm_ctx *L, spm_ctx *const *R, int nr) {
+    if (L->prun_np == 0) return SPM_OK;
+    const PRun<T> *many = static_cast<const PRun<T> *>(L->pruns);
+    const PRun<T>  none{};
+    const unsigned nz = (unsigned)nr, nb = (unsigned)(L->prun_np + 127) / 128;
+    LAUNCH(L, (p_position_run<T, true>), dim3(nb, 1, nz), 128, 0, none, many);
+    LAUNCH(L, (s_phi_scatter_cache<T, true>), dim3((L->prun_cells + 127) / 128, L->prun_np, nz), 128, 0, L->g, none,
+           many);
+    if (lj_cell_list_applies(R[0]->ph)) {  // the same for every run of a grid
+        LAUNCH(L, (p_cells_bin<T, true>), dim3(nb, 1, nz), 128, 0, none, many);
+        LAUNCH(L, (p_forces_cells<T, true>), dim3((L->prun_np + 3) / 4, 1, nz), 128, 0, none, many);
+    } else {
+        for (int r = 0; r < nr; r++) SPM_TRY(lj_forces(R[r], R[r]->ph));
+    }
+    return SPM_OK;
+}
+template <typename T>
+int pool_main_work(spm_ctx *L, spm_ctx *const *R, int nr) {
+    if (L->prun_np == 0) return SPM_OK;
+    const PRun<T> *many = static_cast<const PRun<T> *>(L->pruns);
+    const PRun<T>  none{};
+    const unsigned nz    = (unsigned)nr;
+    bool           noise = false;
+    for (int r = 0; r < nr; r++) noise = noise || prun_of<T>(R[r]).noise;
+    LAUNCH(L, (s_hydro_force_cached<T, true>), dim3(L->prun_np, 1, nz), 256, 0, L->g, none, many);
+    if (noise) LAUNCH(L, p_thermostat_pool<T>, dim3(1, 1, nz), kThermoThreads, 0, many);
+    LAUNCH(L, (s_f_scatter_cached<T, true>), dim3((L->prun_cells + 127) / 128, L->prun_np, nz), 128, 0, L->g, none,
+           many);
     return SPM_OK;
 }
 
@@ -1040,6 +1090,7 @@ int step_ns_runs(spm_ctx *L, spm_ctx *const *R, int nr) {
     // solve; they run on the side stream while the main stream advances zeta.
     // The scatter slots are free here (the previous step consumed them).
     const cudaStream_t side = L->overlap ? L->side : L->st;
+    const bool         pool = L->pruns != nullptr;  // the runs' descriptors are on the device (pool_describe)
     if (L->overlap) {
         SPM_CUDA_CHECK(cudaEventRecord(L->ev_fork, L->st));
         SPM_CUDA_CHECK(cudaStreamWaitEvent(side, L->ev_fork, 0));
@@ -1049,19 +1100,22 @@ int step_ns_runs(spm_ctx *L, spm_ctx *const *R, int nr) {
         L->st                      = side;
         for (int r = 0; r < nr; r++) R[r]->st = side;
         rc = clear_scatter_slots<T>(L);
-        for (int r = 0; r < nr && rc == SPM_OK; r++) {
+        if (rc == SPM_OK && pool) rc = pool_side_work<T>(L, R, nr);
+        for (int r = 0; r < nr && rc == SPM_OK && !pool; r++) {
             spm_ctx *c = R[r];
             if (c->ph.np == 0) continue;
             auto side_work = [&]() -> int {
+                const PRun<T> one = prun_of<T>(c);
                 if (c->rigid())
                     PLAUNCH(c, "r_position", 0.0, r_position, c->rg.nb, 128, 0, c->ph, c->ps, c->rg, c->ts_dev, 0, 0.0,
                             (const double *)nullptr);
                 else
-                    PLAUNCH(c, "p_position", 0.0, p_position, particle_blocks(c), 128, 0, c->ph, c->ps, c->ts_dev, 1);
+                    PLAUNCH(c, "p_position", 0.0, (p_position_run<T, false>), particle_blocks(c), 128, 0, one,
+                            (const PRun<T> *)nullptr);
                 const dim3 sgrid((c->ncells + 127) / 128, c->ph.np);
-                PLAUNCH(c, "s_phi_scatter_cache", stencil_bytes<T>(c, 0), s_phi_scatter_cache<T>, sgrid, 128, 0, c->g,
-                        c->ph, c->ps.x, c->cells, c->ncells, c->real<T>(PHIS), c->err, c->sc_idx, c->sc_w);
-                SPM_TRY(lj_forces(c, c->ph));
+                PLAUNCH(c, "s_phi_scatter_cache", stencil_bytes<T>(c, 0), (s_phi_scatter_cache<T, false>), sgrid, 128,
+                        0, c->g, one, (const PRun<T> *)nullptr);
+                SPM_TRY(lj_forces(c, c->ph, c->rigid()));
                 return SPM_OK;
             };
             rc = side_work();
@@ -1081,30 +1135,27 @@ int step_ns_runs(spm_ctx *L, spm_ctx *const *R, int nr) {
         SPM_TRY(zeta_to_velocity<T>(L, 1, true));
     }
     if (L->overlap) SPM_CUDA_CHECK(cudaStreamWaitEvent(L->st, L->ev_join, 0));  // join
-    for (int r = 0; r < nr; r++) {
+    if (pool) SPM_TRY(pool_main_work<T>(L, R, nr));
+    for (int r = 0; r < nr && !pool; r++) {
         spm_ctx *c = R[r];
         if (c->ph.np == 0) continue;
-        PLAUNCH(c, "s_hydro_force_cached", stencil_bytes<T>(c, 1), s_hydro_force_cached<T>, c->ph.np, 256, 0, c->g,
-                c->ph, c->ps.x, c->ps.v, c->ps.omega, c->cells, c->ncells, c->sc_idx, c->sc_w, c->real<T>(PHIS),
-                c->real<T>(U0), c->real<T>(U1), c->real<T>(U2), c->ps.f_hydro, c->ps.torque_hydro);
+        const PRun<T> one = prun_of<T>(c);
+        PLAUNCH(c, "s_hydro_force_cached", stencil_bytes<T>(c, 1), (s_hydro_force_cached<T, false>), c->ph.np, 256, 0,
+                c->g, one, (const PRun<T> *)nullptr);
         if (c->rigid()) {
             LAUNCH(c, r_collect, c->rg.nb, 128, 0, c->ps, c->rg, c->rfree, 0);
             LAUNCH(c, r_velocity, c->rg.nb, 128, 0, c->ph, c->ps, c->rg, c->rfree, c->ts_dev, 0, 0.0,
                    (const double *)nullptr);
         } else if (c->ph.janus_prop == SPM_JANUS_SQUIRMER) {
             SPM_TRY(slip_loop<T>(c));  // lone runs only; leaves the slip field in UP
-        } else {
-            PLAUNCH(c, "p_velocity", 0.0, p_velocity, particle_blocks(c), 128, 0, c->ph, c->ps, c->ts_dev);
         }
-        // obstacles draw no noise (fluct.cxx:23)
-        if (c->P.kbt > 0.0 && c->ph.janus_prop != SPM_JANUS_OBSTACLE) {
+        if (one.noise) {
             LAUNCH(c, p_thermostat, 1, kThermoThreads, 0, c->ph, c->ps, c->mt, c->rigid() ? c->rg.noise : nullptr);
             if (c->rigid()) LAUNCH(c, r_thermostat, c->rg.nb, 128, 0, c->ph, c->ps, c->rg, c->rfree);
         }
         const dim3 sgrid((c->ncells + 127) / 128, c->ph.np);
-        PLAUNCH(c, "s_f_scatter_cached", stencil_bytes<T>(c, 2), s_f_scatter_cached<T>, sgrid, 128, 0, c->g, c->ph,
-                c->ps.x, c->ps.v, c->ps.omega, c->cells, c->ncells, c->sc_idx, c->sc_w, c->real<T>(PHIS),
-                c->real<T>(U0), c->real<T>(U1), c->real<T>(U2), c->real<T>(UP0), c->real<T>(UP1), c->real<T>(UP2));
+        PLAUNCH(c, "s_f_scatter_cached", stencil_bytes<T>(c, 2), (s_f_scatter_cached<T, false>), sgrid, 128, 0, c->g,
+                one, (const PRun<T> *)nullptr);
     }
     if (L->sns) SPM_TRY(shear_diagnostics<T>(L));  // lone Shear_Navier_Stokes runs
     if ((rc = rigidity_projection<T>(L, nr, 1)) != SPM_OK) return rc;
@@ -1407,6 +1458,7 @@ void destroy_ctx(spm_ctx *c) {
     dev_free(c->le.partial);
     dev_free(c->el.dev);
     dev_free(c->el.partial);
+    dev_free(c->pruns);
     dev_free(c->slip);
     dev_free(c->slip_eps);
     dev_free(c->sns);

@@ -121,9 +121,9 @@ __global__ void __launch_bounds__(W *Split<N>::N1)
 
 // ---------------------------------------------------------------------------
 // Strided complex pass, persistent and TMA-pipelined.
-// The field is a 4D tensor of T: {2*hnz (kz re/im), NY, NX, nfields}.  A tile
-// is W kz-columns x N lines (box {2W, N, 1, 1} on the Y pass, {2W, 1, N, 1}
-// on the X pass); in shared memory both arrive as [n][W] complex.  Each CTA
+// The fields are a 5D tensor of T: {2*hnz (kz re/im), NY, NX, runs, fields} (a
+// pool's runs are one launch).  A tile is W kz-columns x N lines (box {2W, N,
+// 1, 1, 1} on the Y pass, {2W, 1, N, 1, 1} on the X pass); in shared memory both arrive as [n][W] complex.  Each CTA
 // walks its tiles through an S-deep ring of buffers: TMA loads run S-1 tiles
 // ahead of the four-step FFT, results go back with TMA stores from the same
 // buffer.  Columns >= hnz are outside the tensor: loads zero-fill them and
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(W *Split<N>::N1)
 template <typename T, int N, int W, int DIR, int S>
 __global__ void __launch_bounds__(W *Split<N>::N1)
     fft_strided_tma_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant__ CUtensorMap smap,
-                           int axis, int n_outer, int ct_used, int ntiles, const cplx<T> *__restrict__ twN,
+                           int axis, int n_outer, int ct_used, int nruns, int ntiles, const cplx<T> *__restrict__ twN,
                            unsigned int *err, PassPrune pr, unsigned long long wait_ns, int skip_loads) {
     constexpr int  N1         = Split<N>::N1;
     constexpr int  N2         = Split<N>::N2;
@@ -155,11 +155,12 @@ __global__ void __launch_bounds__(W *Split<N>::N1)
     const int c   = tid % W;
     const int g   = tid / W;
     const int n_used = outer_count(n_outer, pr.outer_trn);
-    auto coords = [&](int t, int &c0, int &c1, int &c2, int &c3) {
+    auto coords = [&](int t, int &c0, int &c1, int &c2, int &c3, int &c4) {
         const int ct = t % ct_used, rest = t / ct_used;
         const int o = outer_line(rest % n_used, n_outer, pr.outer_trn), f = rest / n_used;
         c0 = 2 * ct * W;
-        c3 = f;
+        c3 = f % nruns;  // run of a pool
+        c4 = f / nruns;
         if (axis == 1) {
             c1 = 0;
             c2 = o;
@@ -179,14 +180,14 @@ __global__ void __launch_bounds__(W *Split<N>::N1)
     auto load_tile   = [&](int t, int b) {
         if (skip_loads) return;
         last_issued = (t - (int)blockIdx.x) / (int)gridDim.x;
-        int c0, c1, c2, c3;
-        coords(t, c0, c1, c2, c3);
+        int c0, c1, c2, c3, c4;
+        coords(t, c0, c1, c2, c3, c4);
         cplx<T> *dst = buf + (size_t)b * N * W;
         mbar_expect_tx(&full[b], load_bytes);
-        tma_load_4d(dst, &lmap, c0, c1, c2, c3, &full[b]);
+        tma_load_5d(dst, &lmap, c0, c1, c2, c3, c4, &full[b]);
         if (hl < N) {
             const int sh = N - hl;
-            tma_load_4d(dst + (size_t)sh * W, &lmap, c0, c1 + (axis == 1 ? sh : 0), c2 + (axis == 1 ? 0 : sh), c3,
+            tma_load_5d(dst + (size_t)sh * W, &lmap, c0, c1 + (axis == 1 ? sh : 0), c2 + (axis == 1 ? 0 : sh), c3, c4,
                         &full[b]);
         }
     };
@@ -248,12 +249,13 @@ __global__ void __launch_bounds__(W *Split<N>::N1)
         fence_proxy_async();
         __syncthreads();
         if (tid == 0) {
-            int c0, c1, c2, c3;
-            coords(t, c0, c1, c2, c3);
-            tma_store_4d(&smap, c0, c1, c2, c3, B);
+            int c0, c1, c2, c3, c4;
+            coords(t, c0, c1, c2, c3, c4);
+            tma_store_5d(&smap, c0, c1, c2, c3, c4, B);
             if (hs < N) {
                 const int sh = N - hs;
-                tma_store_4d(&smap, c0, c1 + (axis == 1 ? sh : 0), c2 + (axis == 1 ? 0 : sh), c3, B + (size_t)sh * W);
+                tma_store_5d(&smap, c0, c1 + (axis == 1 ? sh : 0), c2 + (axis == 1 ? 0 : sh), c3, c4,
+                             B + (size_t)sh * W);
             }
             bulk_commit();
             // refill the buffer of the previous iteration with the tile S

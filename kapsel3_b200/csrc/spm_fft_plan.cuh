@@ -9,6 +9,11 @@
 
 namespace spm {
 
+// The library's device allocator (spm_api.cu): blocks of the per-device memory
+// pool, whose release neither waits for the device nor unmaps.
+cudaError_t dev_alloc(void **p, size_t bytes);
+void        dev_free(void *p);
+
 template <typename T>
 struct FFTPlan {
     Grid     g{};
@@ -78,10 +83,10 @@ struct FFTPlan {
         return set_smem_attrs();
     }
     void destroy() {
-        cudaFree(tw_x);
-        cudaFree(tw_y);
-        cudaFree(tw_zm);
-        cudaFree(tw_zn);
+        dev_free(tw_x);
+        dev_free(tw_y);
+        dev_free(tw_zm);
+        dev_free(tw_zn);
         tw_x = tw_y = tw_zm = tw_zn = nullptr;
     }
 
@@ -102,15 +107,16 @@ struct FFTPlan {
     }
 
     // Individual passes (exposed for the fused step).
+    // nruns > 1: the same fields of a pool's runs, run_stride_c complex values apart.
     cudaError_t z_r2c(const T *in, cplx<T> *out, int nfields, size_t fs_real, size_t fs_c, cudaStream_t st,
-                      int kz_span = 1 << 30) const {
+                      int kz_span = 1 << 30, int nruns = 1, size_t run_stride_c = 0) const {
         const int nrows = g.nx * g.ny;
         switch (g.nz / 2) {
 #define SPM_ZR2C(MM)                                                                                          \
     case MM: {                                                                                                \
         constexpr int RR = zr_rows<T, MM>();                                                                  \
-        zr_r2c_kernel<T, MM, RR><<<dim3((nrows + RR - 1) / RR, nfields), RR * ZR<MM>::P, 0, st>>>(            \
-            in, out, fs_real, fs_c, nrows, g.hnzp, tw_zm, tw_zn, kz_span);                                    \
+        zr_r2c_kernel<T, MM, RR><<<dim3((nrows + RR - 1) / RR, nfields, nruns), RR * ZR<MM>::P, 0, st>>>(     \
+            in, out, fs_real, fs_c, run_stride_c, nrows, g.hnzp, tw_zm, tw_zn, kz_span);                      \
     } break;
             SPM_ZR2C(4) SPM_ZR2C(8) SPM_ZR2C(16) SPM_ZR2C(32) SPM_ZR2C(64) SPM_ZR2C(128) SPM_ZR2C(256)
 #undef SPM_ZR2C
@@ -119,19 +125,20 @@ struct FFTPlan {
         return cudaGetLastError();
     }
     cudaError_t z_c2r(const cplx<T> *in, T *out, int nfields, size_t fs_c, size_t fs_real, T scale,
-                      cudaStream_t st, int kz_keep = 1 << 30) const {
+                      cudaStream_t st, int kz_keep = 1 << 30, int nruns = 1, size_t run_stride_c = 0) const {
         const int nrows = g.nx * g.ny;
         switch (g.nz / 2) {
 #define SPM_ZC2R(MM)                                                                                          \
     case MM: {                                                                                                \
         constexpr int RR = zr_rows<T, MM>();                                                                  \
-        const dim3    grid((nrows + RR - 1) / RR, nfields);                                                   \
+        const dim3    grid((nrows + RR - 1) / RR, nfields, nruns);                                            \
         if constexpr (c2r_minb<MM>() > 1)                                                                     \
             zr_c2r_kernel_capped<T, MM, RR, c2r_minb<MM>()><<<grid, RR * ZR<MM>::P, 0, st>>>(                 \
-                in, out, fs_c, fs_real, nrows, g.hnzp, tw_zm, tw_zn, scale, kz_keep);                         \
+                in, out, fs_c, fs_real, run_stride_c, nrows, g.hnzp, tw_zm, tw_zn, scale, kz_keep);           \
         else                                                                                                  \
-            zr_c2r_kernel<T, MM, RR><<<grid, RR * ZR<MM>::P, 0, st>>>(in, out, fs_c, fs_real, nrows, g.hnzp,  \
-                                                                      tw_zm, tw_zn, scale, kz_keep);          \
+            zr_c2r_kernel<T, MM, RR><<<grid, RR * ZR<MM>::P, 0, st>>>(in, out, fs_c, fs_real, run_stride_c,   \
+                                                                      nrows, g.hnzp, tw_zm, tw_zn, scale,     \
+                                                                      kz_keep);                               \
     } break;
             SPM_ZC2R(4) SPM_ZC2R(8) SPM_ZC2R(16) SPM_ZC2R(32) SPM_ZC2R(64) SPM_ZC2R(128) SPM_ZC2R(256)
 #undef SPM_ZC2R
@@ -154,23 +161,24 @@ struct FFTPlan {
     int           sm_count    = 148;
 
     template <int DIR>
-    cudaError_t strided_tma(cplx<T> *data, int nfields, size_t fs_c, int axis, cudaStream_t st,
-                            PassPrune pr) const {
+    cudaError_t strided_tma(cplx<T> *data, int nfields, size_t fs_c, int nruns, size_t run_stride_c, int axis,
+                            cudaStream_t st, PassPrune pr) const {
         const int n = axis == 1 ? g.ny : g.nx;
         if (n > 256 || !encode_tiled_fn()) return cudaErrorNotSupported;
         const int outer   = axis == 1 ? g.nx : g.ny;
         const int ct_used = (std::min(pr.kz_cols, g.hnz) + W_T - 1) / W_T;
-        const int ntiles  = nfields * outer_count(outer, pr.outer_trn) * ct_used;
+        const int ntiles  = nfields * nruns * outer_count(outer, pr.outer_trn) * ct_used;
         if (ntiles == 0) return cudaSuccess;
-        const uint64_t dims[4] = {(uint64_t)2 * g.hnz, (uint64_t)g.ny, (uint64_t)g.nx, (uint64_t)nfields};
-        const uint64_t strides[3] = {(uint64_t)2 * g.hnzp * sizeof(T), (uint64_t)g.ny * 2 * g.hnzp * sizeof(T),
-                                     (uint64_t)fs_c * sizeof(cplx<T>)};
+        const uint64_t dims[5] = {(uint64_t)2 * g.hnz, (uint64_t)g.ny, (uint64_t)g.nx, (uint64_t)nruns,
+                                  (uint64_t)nfields};
+        const uint64_t strides[4] = {(uint64_t)2 * g.hnzp * sizeof(T), (uint64_t)g.ny * 2 * g.hnzp * sizeof(T),
+                                     (uint64_t)run_stride_c * sizeof(cplx<T>), (uint64_t)fs_c * sizeof(cplx<T>)};
         // load and store maps: boxes of N lines, or of the pruned line count
         // (two boxes per tile, pruned_box_lines)
         CUtensorMap lmap, smap;
         auto        make = [&](CUtensorMap *m, int lines) {
-            const uint32_t box[4] = {(uint32_t)(2 * W_T), axis == 1 ? (uint32_t)lines : 1u,
-                                     axis == 1 ? 1u : (uint32_t)lines, 1u};
+            const uint32_t box[5] = {(uint32_t)(2 * W_T), axis == 1 ? (uint32_t)lines : 1u,
+                                     axis == 1 ? 1u : (uint32_t)lines, 1u, 1u};
             return make_map<T>(m, data, dims, strides, box);
         };
         if (!make(&lmap, pruned_box_lines(n, pr.line_trn)) || !make(&smap, pruned_box_lines(n, pr.out_trn)))
@@ -184,7 +192,7 @@ struct FFTPlan {
     case NN:                                                                                                   \
         fft_strided_tma_kernel<T, NN, W_T, DIR, S_T>                                                           \
             <<<grid, W_T * Split<NN>::N1, (size_t)S_T * NN * W_T * sizeof(cplx<T>), st>>>(                     \
-                lmap, smap, axis, outer, ct_used, ntiles, tw, err, pr, wait_ns, skip);                         \
+                lmap, smap, axis, outer, ct_used, nruns, ntiles, tw, err, pr, wait_ns, skip);                         \
         break;
             SPM_TMA(8) SPM_TMA(16) SPM_TMA(32) SPM_TMA(64) SPM_TMA(128) SPM_TMA(256)
 #undef SPM_TMA
@@ -192,11 +200,6 @@ struct FFTPlan {
         }
         return cudaGetLastError();
     }
-    template <int DIR>
-    cudaError_t strided_tma(cplx<T> *data, int nfields, size_t fs_c, int axis, cudaStream_t st) const {
-        return strided_tma<DIR>(data, nfields, fs_c, axis, st, PassPrune::full(g.hnz));
-    }
-
     // axis 1 = Y, axis 0 = X
     template <int DIR>
     cudaError_t strided(cplx<T> *data, int nfields, size_t fs_c, int axis, cudaStream_t st, PassPrune pr) const {
@@ -237,7 +240,7 @@ struct FFTPlan {
             const long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)j / (long double)n;
             h[j] = cplx<T>{(T)std::cos(a), (T)std::sin(a)};
         }
-        cudaError_t e = cudaMalloc(dst, sizeof(cplx<T>) * count);
+        cudaError_t e = dev_alloc((void **)dst, sizeof(cplx<T>) * count);
         if (e != cudaSuccess) return e;
         return cudaMemcpy(*dst, h.data(), sizeof(cplx<T>) * count, cudaMemcpyHostToDevice);
     }

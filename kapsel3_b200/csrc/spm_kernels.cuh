@@ -787,6 +787,106 @@ __global__ void s_hydro_force(Grid g, Phys ph, const double *__restrict__ x, con
 }
 
 // ---------------------------------------------------------------------------
+// Particle state (FP64, [Np][3] / [Np][4] arrays).
+// ---------------------------------------------------------------------------
+struct PState {
+    double *x, *x_nopbc, *x_previous, *v, *v_old, *omega, *omega_old;
+    double *q, *q_old;  // [Np][4]: s, v0, v1, v2
+    double *f_hydro, *f_hydro_previous, *torque_hydro, *torque_hydro_previous;
+    double *fr, *fr_previous, *torque_r, *torque_r_previous;
+    double *mdf;        // momentum_depend_fr [Np][3] (particle_solver.cxx:336-432)
+    double *lj_stress;  // [Np] per-particle share of sum f_x r_y (LE stress)
+};
+
+// qvq = q (0, v) q* (qtn_qvq_prod, quaternion.h:189-196); conj: with q*.
+__device__ __forceinline__ void qtn_rotate_d(const double *q, const double *v, double *out, bool conj) {
+    const double s = q[0], a = conj ? -q[1] : q[1], b = conj ? -q[2] : q[2], c = conj ? -q[3] : q[3];
+    const double qs2 = s * s - (a * a + b * b + c * c);
+    const double dot = a * v[0] + b * v[1] + c * v[2];
+    out[0] = qs2 * v[0] + 2.0 * (dot * a + s * (b * v[2] - c * v[1]));
+    out[1] = qs2 * v[1] + 2.0 * (dot * b + s * (c * v[0] - a * v[2]));
+    out[2] = qs2 * v[2] + 2.0 * (dot * c + s * (a * v[1] - b * v[0]));
+}
+
+// self_propulsion (particle_solver.cxx:88-101): a TUMBLER's body-frame force
+// and torque in the space frame (rigid_body_rotation BODY2SPACE).
+__device__ __forceinline__ void self_propulsion_d(const Phys &ph, const double *q, double *f, double *t) {
+    if (ph.janus_prop == 1) {
+        qtn_rotate_d(q, ph.janus_force, f, false);
+        qtn_rotate_d(q, ph.janus_torque, t, false);
+    } else {
+        f[0] = f[1] = f[2] = t[0] = t[1] = t[2] = 0.0;
+    }
+}
+
+// Velocity and angular-velocity update of component d of particle n (Euler at
+// step 0, AB2 after) and the shift of the current forces to the previous ones.
+__device__ __forceinline__ void velocity_update_comp(const Phys &ph, const PState &s, int n, int d, int euler) {
+    const int    sp  = spec_of(ph, n);
+    const double dmy = (euler ? ph.dt : ph.hdt) * ph.imass_s[sp];
+    const double dmr = (euler ? ph.dt : ph.hdt) * ph.imoi_s[sp];
+    double       sf[3], st[3];
+    self_propulsion_d(ph, s.q + 4 * n, sf, st);
+    const double sfd = d == 0 ? sf[0] : d == 1 ? sf[1] : sf[2];
+    const double std = d == 0 ? st[0] : d == 1 ? st[1] : st[2];
+    const int    i   = 3 * n + d;
+    s.v_old[i]       = s.v[i];
+    s.omega_old[i]   = s.omega[i];
+    if (ph.janus_prop == 3) {  // OBSTACLE
+        s.v[i]     = 0.0;
+        s.omega[i] = 0.0;
+    } else if (euler) {
+        s.v[i] += dmy * (s.f_hydro[i] + s.fr[i] + sfd);
+        s.omega[i] += dmr * (s.torque_hydro[i] + s.torque_r[i] + std);
+    } else {
+        s.v[i] += dmy * (2.0 * (s.f_hydro[i] + sfd) + s.fr[i] + s.fr_previous[i]);
+        s.omega[i] += dmr * (2.0 * (s.torque_hydro[i] + std) + s.torque_r[i] + s.torque_r_previous[i]);
+    }
+    s.fr_previous[i]           = s.fr[i];
+    s.fr[i]                    = 0.0;
+    s.f_hydro_previous[i]      = s.f_hydro[i];
+    s.f_hydro[i]               = 0.0;
+    s.torque_r_previous[i]     = s.torque_r[i];
+    s.torque_r[i]              = 0.0;
+    s.torque_hydro_previous[i] = s.torque_hydro[i];
+    s.torque_hydro[i]          = 0.0;
+}
+__device__ __forceinline__ void velocity_update_one(const Phys &ph, const PState &s, int n, int euler) {
+    for (int d = 0; d < 3; d++) velocity_update_comp(ph, s, n, d, euler);
+}
+
+// ---------------------------------------------------------------------------
+// What the step's particle kernels need of one run.  A lone run passes it by
+// value; the runs of a pool keep theirs in a device array and are one launch,
+// blockIdx.z the run (POOL).  A launch per run was most of a pool's step: at
+// 64^3 with 8 runs of 75 colloids 56 of its 97 launches, 336 of 641 us.
+// ---------------------------------------------------------------------------
+template <typename T>
+struct PRun {
+    Phys          ph;
+    PState        ps;
+    const int    *cells;   // Sekibun stencil
+    int           ncells;
+    int           vel;     // s_hydro_force_cached also updates the velocities
+    int           noise;   // thermostat on
+    T            *phi_sum, *u0, *u1, *u2, *f0, *f1, *f2;
+    int          *sc_idx;  // stencil cache
+    double       *sc_w;
+    int          *lj_count, *lj_cell_of, *lj_bins, lj_ncell;  // LJ cell list
+    const int    *rid;     // rigid bodies, or null
+    double       *f_lo;
+    const int    *ts;
+    unsigned int *mt, *err;
+};
+template <bool POOL, typename T>
+__device__ __forceinline__ const PRun<T> &prun(const PRun<T> &one, const PRun<T> *__restrict__ many) {
+    if constexpr (POOL)
+        return many[blockIdx.z];
+    else
+        return one;
+}
+
+// ---------------------------------------------------------------------------
 // Stencil cache of the step.  The phi scatter evaluates, for every (particle,
 // Sekibun cell), the grid index and the profile weight Phi; the hydrodynamic
 // force and the phi*v_p scatter of the same step (same positions) read them
@@ -809,42 +909,44 @@ __device__ __forceinline__ void cell_offset(const Grid &g, int cell_packed, cons
     for (int d = 0; d < 3; d++) r[d] = (double)c[d] * g.dx - res[d];
 }
 
-template <typename T>
-__global__ void s_phi_scatter_cache(Grid g, Phys ph, const double *__restrict__ x, const int *__restrict__ cells,
-                                    int ncells, T *__restrict__ phi_sum, unsigned int *err, int *__restrict__ sc_idx,
-                                    double *__restrict__ sc_w) {
+template <typename T, bool POOL>
+__global__ void s_phi_scatter_cache(Grid g, const __grid_constant__ PRun<T> one, const PRun<T> *__restrict__ many) {
+    const PRun<T> &R = prun<POOL>(one, many);
     const int p = blockIdx.y;
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= ph.np || m >= ncells) return;
-    const size_t o     = (size_t)p * ncells + m;
-    const double xp[3] = {x[3 * p], x[3 * p + 1], x[3 * p + 2]};
-    if (!particle_in_box(ph, xp)) {
-        if (m == 0) atomicOr(err, (unsigned)SPM_DEVERR_PARTICLE_OUT_OF_BOX);
-        sc_idx[o] = -1;
+    if (p >= R.ph.np || m >= R.ncells) return;
+    const size_t  o     = (size_t)p * R.ncells + m;
+    const double *x     = R.ps.x;
+    const double  xp[3] = {x[3 * p], x[3 * p + 1], x[3 * p + 2]};
+    if (!particle_in_box(R.ph, xp)) {
+        if (m == 0) atomicOr(R.err, (unsigned)SPM_DEVERR_PARTICLE_OUT_OF_BOX);
+        R.sc_idx[o] = -1;
         return;
     }
     StencilPoint s;
-    stencil_point(g, ph, xp, cells[m], s);
-    const double v = phi_prof(s.dist, ph.radius, ph.hxi, g.dx);
-    sc_idx[o]      = v != 0.0 ? (int)s.idx : -1;
-    sc_w[o]        = v;
-    if (v != 0.0) atomicAdd(&phi_sum[s.idx], (T)v);
+    stencil_point(g, R.ph, xp, R.cells[m], s);
+    const double v = phi_prof(s.dist, R.ph.radius, R.ph.hxi, g.dx);
+    R.sc_idx[o]    = v != 0.0 ? (int)s.idx : -1;
+    R.sc_w[o]      = v;
+    if (v != 0.0) atomicAdd(&R.phi_sum[s.idx], (T)v);
 }
 
 // Calc_f_hydro_correct_precision from the stencil cache (same sums as
 // s_hydro_force).
-template <typename T>
-__global__ void s_hydro_force_cached(Grid g, Phys ph, const double *__restrict__ x, const double *__restrict__ v,
-                                     const double *__restrict__ w, const int *__restrict__ cells, int ncells,
-                                     const int *__restrict__ sc_idx, const double *__restrict__ sc_w,
-                                     const T *__restrict__ phi_sum, const T *__restrict__ u0,
-                                     const T *__restrict__ u1, const T *__restrict__ u2, double *__restrict__ f_hydro,
-                                     double *__restrict__ torque_hydro) {
-    const int p = blockIdx.x;
+template <typename T, bool POOL>
+__global__ void s_hydro_force_cached(Grid g, const __grid_constant__ PRun<T> one, const PRun<T> *__restrict__ many) {
+    const PRun<T> &R = prun<POOL>(one, many);
+    const Phys    &ph = R.ph;
+    const int      p  = blockIdx.x;
     if (p >= ph.np) return;
-    const double xp[3] = {x[3 * p], x[3 * p + 1], x[3 * p + 2]};
-    const double vp[3] = {v[3 * p], v[3 * p + 1], v[3 * p + 2]};
-    const double op[3] = {w[3 * p], w[3 * p + 1], w[3 * p + 2]};
+    const PState &s      = R.ps;
+    const int     ncells = R.ncells;
+    const int *__restrict__ sc_idx = R.sc_idx, *__restrict__ cells = R.cells;
+    const double *__restrict__ sc_w = R.sc_w;
+    const T *__restrict__ phi_sum = R.phi_sum, *__restrict__ u0 = R.u0, *__restrict__ u1 = R.u1, *__restrict__ u2 = R.u2;
+    const double xp[3] = {s.x[3 * p], s.x[3 * p + 1], s.x[3 * p + 2]};
+    const double vp[3] = {s.v[3 * p], s.v[3 * p + 1], s.v[3 * p + 2]};
+    const double op[3] = {s.omega[3 * p], s.omega[3 * p + 1], s.omega[3 * p + 2]};
     double       res[3];
     particle_residue(g, xp, res);
     double acc[6] = {0, 0, 0, 0, 0, 0};
@@ -897,11 +999,15 @@ __global__ void s_hydro_force_cached(Grid g, Phys ph, const double *__restrict__
         }
     }
     block_sum6(acc);
-    if (threadIdx.x == 0) {
+    // component d by lane d of the first warp, which holds the sums
+    if (threadIdx.x < 3) {
+        const int    d   = threadIdx.x;
         const double dmy = -ph.dx3 * ph.rho / ph.dt;
-        for (int d = 0; d < 3; d++) f_hydro[3 * p + d] = dmy * acc[d];
-        if (ph.rotation)
-            for (int d = 0; d < 3; d++) torque_hydro[3 * p + d] = dmy * acc[3 + d];
+        s.f_hydro[3 * p + d] = dmy * (d == 0 ? acc[0] : d == 1 ? acc[1] : acc[2]);
+        if (ph.rotation) s.torque_hydro[3 * p + d] = dmy * (d == 0 ? acc[3] : d == 1 ? acc[4] : acc[5]);
+        // the velocities need nothing but this particle's own forces: updating
+        // them here is one launch (6 to 7 us of latency on B200) fewer
+        if (R.vel) velocity_update_comp(ph, s, p, d, *R.ts == 0);
     }
 }
 
@@ -912,48 +1018,34 @@ __global__ void s_hydro_force_cached(Grid g, Phys ph, const double *__restrict__
 // integrand of the hydrodynamic force.  f is zero wherever no profile
 // reaches, so the forward z pass of f reads three fields instead of the
 // seven (up, u, phi) of forming f on the fly.
-template <typename T>
-__global__ void s_f_scatter_cached(Grid g, Phys ph, const double *__restrict__ x, const double *__restrict__ v,
-                                   const double *__restrict__ w, const int *__restrict__ cells, int ncells,
-                                   const int *__restrict__ sc_idx, const double *__restrict__ sc_w,
-                                   const T *__restrict__ phi_sum, const T *__restrict__ u0, const T *__restrict__ u1,
-                                   const T *__restrict__ u2, T *__restrict__ f0, T *__restrict__ f1,
-                                   T *__restrict__ f2) {
+template <typename T, bool POOL>
+__global__ void s_f_scatter_cached(Grid g, const __grid_constant__ PRun<T> one, const PRun<T> *__restrict__ many) {
+    const PRun<T> &R = prun<POOL>(one, many);
     const int p = blockIdx.y;
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= ph.np || m >= ncells) return;
-    const size_t o  = (size_t)p * ncells + m;
-    const int    id = sc_idx[o];
+    if (p >= R.ph.np || m >= R.ncells) return;
+    const size_t o  = (size_t)p * R.ncells + m;
+    const int    id = R.sc_idx[o];
     if (id < 0) return;
+    const double *x = R.ps.x, *v = R.ps.v;
     const double xp[3] = {x[3 * p], x[3 * p + 1], x[3 * p + 2]};
     double       res[3], r[3];
     particle_residue(g, xp, res);
-    cell_offset(g, cells[m], res, r);
-    const double ps  = (double)phi_sum[id];
-    const double wgt = sc_w[o] / (ps > 1.0 ? ps : 1.0);
+    cell_offset(g, R.cells[m], res, r);
+    const double ps  = (double)R.phi_sum[id];
+    const T      a0 = R.u0[id], a1 = R.u1[id], a2 = R.u2[id];  // before the atomics, which could alias them
+    const double wgt = R.sc_w[o] / (ps > 1.0 ? ps : 1.0);
     double       vs[3] = {v[3 * p], v[3 * p + 1], v[3 * p + 2]};
-    if (ph.rotation) {
-        const double *om = w + 3 * p;
+    if (R.ph.rotation) {
+        const double *om = R.ps.omega + 3 * p;
         vs[0] += om[1] * r[2] - om[2] * r[1];
         vs[1] += om[2] * r[0] - om[0] * r[2];
         vs[2] += om[0] * r[1] - om[1] * r[0];
     }
-    atomicAdd(&f0[id], (T)((vs[0] - (double)u0[id]) * wgt));
-    atomicAdd(&f1[id], (T)((vs[1] - (double)u1[id]) * wgt));
-    atomicAdd(&f2[id], (T)((vs[2] - (double)u2[id]) * wgt));
+    atomicAdd(&R.f0[id], (T)((vs[0] - (double)a0) * wgt));
+    atomicAdd(&R.f1[id], (T)((vs[1] - (double)a1) * wgt));
+    atomicAdd(&R.f2[id], (T)((vs[2] - (double)a2) * wgt));
 }
-
-// ---------------------------------------------------------------------------
-// Particle state (FP64, [Np][3] / [Np][4] arrays).
-// ---------------------------------------------------------------------------
-struct PState {
-    double *x, *x_nopbc, *x_previous, *v, *v_old, *omega, *omega_old;
-    double *q, *q_old;  // [Np][4]: s, v0, v1, v2
-    double *f_hydro, *f_hydro_previous, *torque_hydro, *torque_hydro_previous;
-    double *fr, *fr_previous, *torque_r, *torque_r_previous;
-    double *mdf;        // momentum_depend_fr [Np][3] (particle_solver.cxx:336-432)
-    double *lj_stress;  // [Np] per-particle share of sum f_x r_y (LE stress)
-};
 
 __device__ __forceinline__ void qtn_prod_d(const double *qa, const double *qb, double alpha, double *q) {
     q[0] = alpha * (qa[0] * qb[0] - (qa[1] * qb[1] + qa[2] * qb[2] + qa[3] * qb[3]));
@@ -978,10 +1070,8 @@ __device__ __forceinline__ void qtn_normalize_d(double *q) {
 // wrap = 0 leaves the periodic wrap to p_le_wrap (Lees-Edwards image).
 // The Euler start (ts == 0) is read from the run's device step counter, so a
 // captured step graph serves every step.
-__global__ void p_position(Phys ph, PState s, const int *__restrict__ ts_dev, int wrap) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void position_one(const Phys &ph, const PState &s, int n, int euler, int wrap) {
     if (n >= ph.np || ph.janus_prop == 3) return;  // OBSTACLE: fixed (particle_solver.cxx:44)
-    const int euler = *ts_dev == 0;
     for (int d = 0; d < 3; d++) {
         const int i       = 3 * n + d;
         s.x_previous[i]   = s.x[i];
@@ -1006,6 +1096,20 @@ __global__ void p_position(Phys ph, PState s, const int *__restrict__ ts_dev, in
         }
         qtn_normalize_d(q);
     }
+}
+
+__global__ void p_position(Phys ph, PState s, const int *__restrict__ ts_dev, int wrap) {
+    position_one(ph, s, blockIdx.x * blockDim.x + threadIdx.x, *ts_dev == 0, wrap);
+}
+// The same for the Navier_Stokes step, which also clears the counts of the LJ
+// cell list for the binning that follows.
+template <typename T, bool POOL>
+__global__ void p_position_run(const __grid_constant__ PRun<T> one, const PRun<T> *__restrict__ many) {
+    const PRun<T> &R = prun<POOL>(one, many);
+    const int      n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (R.lj_count)
+        for (int c = n; c < R.lj_ncell; c += gridDim.x * blockDim.x) R.lj_count[c] = 0;
+    position_one(R.ph, R.ps, n, *R.ts == 0, 1);
 }
 
 // Lennard-Jones magnitude / r (Lennard_Jones_f, interaction.h:160-199).
@@ -1192,18 +1296,21 @@ __device__ __forceinline__ int lj_cell_axis(const Phys &ph, double x, int d, boo
 
 // One thread per particle: its cell, and a slot in the cell's bin (count[]
 // zeroed before the launch).
-__global__ void p_cells_bin(Phys ph, const double *__restrict__ x, int *__restrict__ count,
-                            int *__restrict__ cell_of, int *__restrict__ bins, unsigned int *err) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= ph.np) return;
+template <typename T, bool POOL>
+__global__ void p_cells_bin(const __grid_constant__ PRun<T> one, const PRun<T> *__restrict__ many) {
+    const PRun<T> &R = prun<POOL>(one, many);
+    const Phys    &ph = R.ph;
+    const int      n  = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= ph.np || !ph.lj_on || ph.janus_prop == 3) return;
+    const double *x  = R.ps.x;
     bool      bad = false;
     const int c   = (lj_cell_axis(ph, x[3 * n], 0, bad) * ph.lc[1] + lj_cell_axis(ph, x[3 * n + 1], 1, bad)) *
                       ph.lc[2] +
                   lj_cell_axis(ph, x[3 * n + 2], 2, bad);
-    if (bad && err) atomicOr(err, SPM_DEVERR_PARTICLE_OUT_OF_BOX);
-    cell_of[n]       = c;
-    const int slot   = atomicAdd(&count[c], 1);
-    if (slot < kLjBin) bins[(size_t)c * kLjBin + slot] = n;
+    if (bad && R.err) atomicOr(R.err, SPM_DEVERR_PARTICLE_OUT_OF_BOX);
+    R.lj_cell_of[n]  = c;
+    const int slot   = atomicAdd(&R.lj_count[c], 1);
+    if (slot < kLjBin) R.lj_bins[(size_t)c * kLjBin + slot] = n;
 }
 
 // The next particle index above `last` in cell c (np when none): the bin's
@@ -1238,8 +1345,14 @@ __device__ __forceinline__ int lj_next_in_cell(const Phys &ph, int c, int last, 
 // Beads of rigid bodies (rid != null): pairs within one body are skipped
 // (rigid_chain, interaction.h:18-24), and f_lo[n] receives the force on n
 // from the pairs where n is the lower index (the bodies' torques need it).
-__global__ void p_forces_cells(Phys ph, PState s, const int *__restrict__ count, const int *__restrict__ cell_of,
-                               const int *__restrict__ bins, const int *__restrict__ rid, double *__restrict__ f_lo) {
+template <typename T, bool POOL>
+__global__ void p_forces_cells(const __grid_constant__ PRun<T> one, const PRun<T> *__restrict__ many) {
+    const PRun<T> &R  = prun<POOL>(one, many);
+    const Phys    &ph = R.ph;
+    const PState  &s  = R.ps;
+    const int *__restrict__ count = R.lj_count, *__restrict__ cell_of = R.lj_cell_of, *__restrict__ bins = R.lj_bins;
+    const int *__restrict__ rid  = R.rid;
+    double *__restrict__ f_lo    = R.f_lo;
     const int lane = threadIdx.x & 31;
     const int n    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (n >= ph.np) return;
@@ -1297,60 +1410,6 @@ __global__ void p_forces_cells(Phys ph, PState s, const int *__restrict__ count,
 
 // MD_solver_velocity_Euler / _AB2_hydro (particle_solver.cxx:103-142,
 // 239-281) followed by reset_Forces (particle_solver.cxx:11-37).
-// Velocity / angular-velocity update of particle n (Euler at step 0, AB2
-// after) and the shift of the current forces to the previous ones.
-// qvq = q (0, v) q* (qtn_qvq_prod, quaternion.h:189-196); conj: with q*.
-__device__ __forceinline__ void qtn_rotate_d(const double *q, const double *v, double *out, bool conj) {
-    const double s = q[0], a = conj ? -q[1] : q[1], b = conj ? -q[2] : q[2], c = conj ? -q[3] : q[3];
-    const double qs2 = s * s - (a * a + b * b + c * c);
-    const double dot = a * v[0] + b * v[1] + c * v[2];
-    out[0] = qs2 * v[0] + 2.0 * (dot * a + s * (b * v[2] - c * v[1]));
-    out[1] = qs2 * v[1] + 2.0 * (dot * b + s * (c * v[0] - a * v[2]));
-    out[2] = qs2 * v[2] + 2.0 * (dot * c + s * (a * v[1] - b * v[0]));
-}
-
-// self_propulsion (particle_solver.cxx:88-101): a TUMBLER's body-frame force
-// and torque in the space frame (rigid_body_rotation BODY2SPACE).
-__device__ __forceinline__ void self_propulsion_d(const Phys &ph, const double *q, double *f, double *t) {
-    if (ph.janus_prop == 1) {
-        qtn_rotate_d(q, ph.janus_force, f, false);
-        qtn_rotate_d(q, ph.janus_torque, t, false);
-    } else {
-        f[0] = f[1] = f[2] = t[0] = t[1] = t[2] = 0.0;
-    }
-}
-
-__device__ __forceinline__ void velocity_update_one(const Phys &ph, const PState &s, int n, int euler) {
-    const int    sp  = spec_of(ph, n);
-    const double dmy = (euler ? ph.dt : ph.hdt) * ph.imass_s[sp];
-    const double dmr = (euler ? ph.dt : ph.hdt) * ph.imoi_s[sp];
-    double       sf[3], st[3];
-    self_propulsion_d(ph, s.q + 4 * n, sf, st);
-    for (int d = 0; d < 3; d++) {
-        const int i      = 3 * n + d;
-        s.v_old[i]       = s.v[i];
-        s.omega_old[i]   = s.omega[i];
-        if (ph.janus_prop == 3) {  // OBSTACLE
-            s.v[i]     = 0.0;
-            s.omega[i] = 0.0;
-        } else if (euler) {
-            s.v[i] += dmy * (s.f_hydro[i] + s.fr[i] + sf[d]);
-            s.omega[i] += dmr * (s.torque_hydro[i] + s.torque_r[i] + st[d]);
-        } else {
-            s.v[i] += dmy * (2.0 * (s.f_hydro[i] + sf[d]) + s.fr[i] + s.fr_previous[i]);
-            s.omega[i] += dmr * (2.0 * (s.torque_hydro[i] + st[d]) + s.torque_r[i] + s.torque_r_previous[i]);
-        }
-        s.fr_previous[i]           = s.fr[i];
-        s.fr[i]                    = 0.0;
-        s.f_hydro_previous[i]      = s.f_hydro[i];
-        s.f_hydro[i]               = 0.0;
-        s.torque_r_previous[i]     = s.torque_r[i];
-        s.torque_r[i]              = 0.0;
-        s.torque_hydro_previous[i] = s.torque_hydro[i];
-        s.torque_hydro[i]          = 0.0;
-    }
-}
-
 __global__ void p_velocity(Phys ph, PState s, const int *__restrict__ ts_dev) {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= ph.np) return;
@@ -1427,8 +1486,7 @@ __device__ __forceinline__ unsigned int mt_twist_word(const unsigned int *mt, in
 }
 // noise != null (rigid bodies): the six normals of particle n go to
 // noise[6 n ..], nothing is applied (r_thermostat applies them per body).
-__global__ void __launch_bounds__(kThermoThreads) p_thermostat(Phys ph, PState s, unsigned int *mt_g,
-                                                               double *noise) {
+__device__ __forceinline__ void thermostat_run(const Phys &ph, const PState &s, unsigned int *mt_g, double *noise) {
     __shared__ unsigned int mt[624];
     __shared__ double       uni[624 + 1];  // the carried uniform, then this round's outputs
     __shared__ int          wsum[kThermoThreads / 32];
@@ -1522,6 +1580,16 @@ __global__ void __launch_bounds__(kThermoThreads) p_thermostat(Phys ph, PState s
     }
     for (int i = tid; i < 624; i += blockDim.x) mt_g[i] = mt[i];
     if (tid == 0) mt_g[624] = (unsigned int)sh_mti;
+}
+__global__ void __launch_bounds__(kThermoThreads) p_thermostat(Phys ph, PState s, unsigned int *mt_g,
+                                                               double *noise) {
+    thermostat_run(ph, s, mt_g, noise);
+}
+// The runs of a pool, one block each.
+template <typename T>
+__global__ void __launch_bounds__(kThermoThreads) p_thermostat_pool(const PRun<T> *__restrict__ many) {
+    const PRun<T> &R = many[blockIdx.z];
+    if (R.noise) thermostat_run(R.ph, R.ps, R.mt, nullptr);
 }
 
 

@@ -63,16 +63,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, unsign
     return false;
 }
 
-// 4D tiled TMA load global -> shared, completion counted on `bar`.
-__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3,
-                                            uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
-        "%5}], [%6];" ::"r"(smem_addr(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_addr(bar))
-        : "memory");
-}
-
 // 5D tiled TMA load global -> shared, completion counted on `bar`.
 __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4,
                                             uint64_t *bar) {
@@ -83,12 +73,12 @@ __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
-// 4D tiled TMA store shared -> global (bulk async group).
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, int c0, int c1, int c2, int c3,
+// 5D tiled TMA store shared -> global (bulk async group).
+__device__ __forceinline__ void tma_store_5d(const CUtensorMap *map, int c0, int c1, int c2, int c3, int c4,
                                              const void *src) {
-    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(
+    asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4, %5}], [%6];" ::"l"(
                      reinterpret_cast<uint64_t>(map)),
-                 "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_addr(src))
+                 "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_addr(src))
                  : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }

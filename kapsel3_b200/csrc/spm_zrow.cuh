@@ -279,7 +279,7 @@ constexpr int zr_rows() {
 // allowed); inputs kz >= kz_keep read as zero.
 template <typename T, int M, int R>
 __device__ __forceinline__ void zr_c2r_rows(unsigned char *smem, const cplx<T> *in, T *out, size_t field_stride_c,
-                                            size_t field_stride_real, int nrows, int hnzp,
+                                            size_t field_stride_real, size_t run_stride_c, int nrows, int hnzp,
                                             const cplx<T> *__restrict__ twM, const cplx<T> *__restrict__ twN, T scale,
                                             int kz_keep) {
     constexpr int P = ZR<M>::P, Q = ZR<M>::Q, J = ZR<M>::J, BPT = ZR<M>::BPT;
@@ -287,8 +287,9 @@ __device__ __forceinline__ void zr_c2r_rows(unsigned char *smem, const cplx<T> *
     const int  t   = threadIdx.x % P;
     const int  row = blockIdx.x * R + r;
     const bool ok  = row < nrows;
-    const cplx<T> *rin = in + (size_t)blockIdx.y * field_stride_c + (size_t)(ok ? row : 0) * hnzp;
-    T *rout            = out + (size_t)blockIdx.y * field_stride_real + (size_t)(ok ? row : 0) * 2 * hnzp;
+    const size_t   ro  = (size_t)blockIdx.z * run_stride_c;  // run of a batched pool
+    const cplx<T> *rin = in + ro + (size_t)blockIdx.y * field_stride_c + (size_t)(ok ? row : 0) * hnzp;
+    T *rout            = out + 2 * ro + (size_t)blockIdx.y * field_stride_real + (size_t)(ok ? row : 0) * 2 * hnzp;
     cplx<T>       *S   = reinterpret_cast<cplx<T> *>(smem + r * ZRSmem<T, M>::blk);
     int     a[2];
     cplx<T> wb[2], kv[2][J], xn, z[BPT][Q];
@@ -311,35 +312,38 @@ __device__ __forceinline__ void zr_c2r_rows(unsigned char *smem, const cplx<T> *
 }
 template <typename T, int M, int R>
 __global__ void __launch_bounds__(R *ZR<M>::P)
-    zr_c2r_kernel(const cplx<T> *in, T *out, size_t field_stride_c, size_t field_stride_real, int nrows, int hnzp,
-                  const cplx<T> *__restrict__ twM, const cplx<T> *__restrict__ twN, T scale, int kz_keep) {
+    zr_c2r_kernel(const cplx<T> *in, T *out, size_t field_stride_c, size_t field_stride_real, size_t run_stride_c,
+                  int nrows, int hnzp, const cplx<T> *__restrict__ twM, const cplx<T> *__restrict__ twN, T scale, int kz_keep) {
     __shared__ __align__(16) unsigned char smem[R * ZRSmem<T, M>::blk];
-    zr_c2r_rows<T, M, R>(smem, in, out, field_stride_c, field_stride_real, nrows, hnzp, twM, twN, scale, kz_keep);
+    zr_c2r_rows<T, M, R>(smem, in, out, field_stride_c, field_stride_real, run_stride_c, nrows, hnzp, twM, twN, scale,
+                         kz_keep);
 }
 // The same pass with the registers capped for MINB resident CTAs per SM.
 template <typename T, int M, int R, int MINB>
 __global__ void __launch_bounds__(R *ZR<M>::P, MINB)
-    zr_c2r_kernel_capped(const cplx<T> *in, T *out, size_t field_stride_c, size_t field_stride_real, int nrows,
-                         int hnzp, const cplx<T> *__restrict__ twM, const cplx<T> *__restrict__ twN, T scale,
+    zr_c2r_kernel_capped(const cplx<T> *in, T *out, size_t field_stride_c, size_t field_stride_real,
+                         size_t run_stride_c, int nrows, int hnzp, const cplx<T> *__restrict__ twM, const cplx<T> *__restrict__ twN, T scale,
                          int kz_keep) {
     __shared__ __align__(16) unsigned char smem[R * ZRSmem<T, M>::blk];
-    zr_c2r_rows<T, M, R>(smem, in, out, field_stride_c, field_stride_real, nrows, hnzp, twM, twN, scale, kz_keep);
+    zr_c2r_rows<T, M, R>(smem, in, out, field_stride_c, field_stride_real, run_stride_c, nrows, hnzp, twM, twN, scale,
+                         kz_keep);
 }
 
 // Forward z pass: real rows -> complex rows (in place allowed); outputs kz >=
 // kz_span are not written.
 template <typename T, int M, int R>
 __global__ void __launch_bounds__(R *ZR<M>::P)
-    zr_r2c_kernel(const T *in, cplx<T> *out, size_t field_stride_real, size_t field_stride_c, int nrows, int hnzp,
-                  const cplx<T> *__restrict__ twM, const cplx<T> *__restrict__ twN, int kz_span) {
+    zr_r2c_kernel(const T *in, cplx<T> *out, size_t field_stride_real, size_t field_stride_c, size_t run_stride_c,
+                  int nrows, int hnzp, const cplx<T> *__restrict__ twM, const cplx<T> *__restrict__ twN, int kz_span) {
     constexpr int P = ZR<M>::P, Q = ZR<M>::Q, J = ZR<M>::J, BPT = ZR<M>::BPT;
     __shared__ __align__(16) unsigned char smem[R * ZRSmem<T, M>::blk];
     const int  r   = threadIdx.x / P;
     const int  t   = threadIdx.x % P;
     const int  row = blockIdx.x * R + r;
     const bool ok  = row < nrows;
-    const T   *rin  = in + (size_t)blockIdx.y * field_stride_real + (size_t)(ok ? row : 0) * 2 * hnzp;
-    cplx<T>   *rout = out + (size_t)blockIdx.y * field_stride_c + (size_t)(ok ? row : 0) * hnzp;
+    const size_t ro = (size_t)blockIdx.z * run_stride_c;  // run of a batched pool
+    const T   *rin  = in + 2 * ro + (size_t)blockIdx.y * field_stride_real + (size_t)(ok ? row : 0) * 2 * hnzp;
+    cplx<T>   *rout = out + ro + (size_t)blockIdx.y * field_stride_c + (size_t)(ok ? row : 0) * hnzp;
     cplx<T>   *S    = reinterpret_cast<cplx<T> *>(smem + r * ZRSmem<T, M>::blk);
     using V2        = typename vec2_of<T>::type;
     int     a[2];
