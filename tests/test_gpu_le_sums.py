@@ -30,3 +30,26 @@ def test_stress_sums(gpu, n, side):
     want = np.array([oracle.stress[k] for k in ("shear_rate", "strain", "lj", "hydro_old", "hydro_new", "reynolds",
                                                 "fluid", "apparent")])
     assert np.abs(st - want).max() <= 1e-10 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("shape,n", [((4, 5, 4), 0), ((5, 4, 6), 1), ((6, 5, 5), 17)])
+def test_step_on_other_boxes(gpu, shape, n):
+    """Boxes that are not cubes, across a remap of the strain (|gamma| reaches
+    NX / NY), with and without particles: zeta of every mode, FP64."""
+    cfg = SPMConfig(npx=shape[0], npy=shape[1], npz=shape[2], n_particles=n, a=2.0, a_xi=1.0, dt=0.1, equation=EQ_LE,
+                    shear_rate=1.3, lj_truncate="ON" if n > 1 else "NONE")
+    parts = make_particles(cfg, seed=n, v_sd=1e-3, random_orientation=True)
+    oracle = OracleSPMLE(cfg, parts)
+    rng = np.random.default_rng(5)
+    u = 1e-2 * rng.normal(size=(3,) + cfg.shape)
+    oracle.zeta, oracle.uk_dc = oracle.u_k2zeta_k(oracle.solenoidal_uk(oracle.truncate(oracle.fft(u))))
+    with SPMRun(cfg) as run:
+        run.initialize(parts)
+        run.set_zeta(oracle.zeta, oracle.uk_dc)
+        steps = int(np.ceil(cfg.shape[0] / cfg.shape[1] / 0.13)) + 2
+        run.step(steps)
+        zeta, _ = run.zeta()
+    for _ in range(steps):
+        oracle.step()
+    assert abs(oracle.gamma) < cfg.shape[0] / cfg.shape[1]
+    assert np.linalg.norm(zeta - oracle.zeta) <= 1e-11 * np.linalg.norm(oracle.zeta)
