@@ -311,7 +311,8 @@ __device__ __forceinline__ int wrap_x(double v, int nx) { return (int)fmod(v, (d
 // power of two) and its row's shift without a division or fmod: with 64-bit
 // divisions per cell this kernel took 29 us and the average gradient apart 19
 // us at 128^3 FP32 on B200, 24 us for both here.  (A warp per row, one shift
-// for its cells, has too few loads in flight: 24 us.)  The cells also add up
+// for its cells, takes as long here and 36 against 28 us in r_le_force_add.)
+// The cells also add up
 // Calc_shear_rate_eff's average gradient of the oblique x velocity (sp_3d_ns.h:
 // 166-203): one FP64 partial per CTA, summed by k_le_shear_rate.
 template <typename T>
