@@ -606,7 +606,7 @@ double pass_elems_rw(spm_ctx *c, int nf, int axis, const PassPrune &pr) {
     const Grid &g     = c->g;
     const int   n     = axis == 1 ? g.ny : g.nx;
     const int   outer = axis == 1 ? g.nx : g.ny;
-    const int   wk    = (c->use_tma && n <= 256) ? FFTPlan<T>::W_T : FFTPlan<T>::W;
+    const int   wk    = c->use_tma ? FFTPlan<T>::w_t(n) : FFTPlan<T>::W;
     const int   cols  = std::min(g.hnz, (std::min(pr.kz_cols, g.hnz) + wk - 1) / wk * wk);
     const int   hl    = pruned_box_lines(n, pr.line_trn);
     const int   hs    = pruned_box_lines(n, pr.out_trn);

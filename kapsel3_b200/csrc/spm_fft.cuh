@@ -43,10 +43,12 @@ struct PassPrune {
     int out_trn;    // > 0: only output lines with |K(n)| < out_trn are needed
     static PassPrune full(int hnz) { return PassPrune{hnz, 0, 0, hnz, 0}; }
 };
-// Lines a TMA box of a pruned pass covers: two boxes of h lines at 0 and
-// N - h hold every line with |K| < trn (h = trn), one box of N lines
-// otherwise.
-__host__ __device__ __forceinline__ int pruned_box_lines(int n, int trn) { return (trn > 0 && 2 * trn < n) ? trn : n; }
+// Lines a TMA box of a pass covers: two boxes of h lines at 0 and N - h hold
+// every line with |K| < trn (h = trn); an unpruned pass is one box of N lines,
+// two halves where N is past the 256 a box can have.
+__host__ __device__ __forceinline__ int pruned_box_lines(int n, int trn) {
+    return (trn > 0 && 2 * trn < n) ? trn : n > 256 ? n / 2 : n;
+}
 
 __host__ __device__ __forceinline__ int signed_mode(int n, int len) { return n > len / 2 ? n - len : n; }
 __host__ __device__ __forceinline__ int outer_count(int n_outer, int outer_trn) {
@@ -197,12 +199,18 @@ __global__ void __launch_bounds__(W *Split<N>::N1)
             if (t < ntiles) load_tile(t, b);
         }
     }
-    // the step-1 twiddles of this thread's n1 = g are the same for every tile
-    cplx<T> tw1[N2];
+    // the step-1 twiddles of this thread's n1 = g are the same for every tile; 32
+    // of them would not fit the registers beside a 32-point transform
+    constexpr bool kTwReg = N2 <= 16;
+    cplx<T>        tw1[kTwReg ? N2 : 1];
+    auto           twiddle = [&](int k1) {
+        cplx<T> w = twN[(g * k1) & (N - 1)];
+        if (DIR > 0) w.im = -w.im;
+        return w;
+    };
+    if constexpr (kTwReg) {
 #pragma unroll
-    for (int k1 = 1; k1 < N2; k1++) {
-        tw1[k1] = twN[(g * k1) & (N - 1)];
-        if (DIR > 0) tw1[k1].im = -tw1[k1].im;
+        for (int k1 = 1; k1 < N2; k1++) tw1[k1] = twiddle(k1);
     }
     int  it      = 0;
     bool stopped = false;
@@ -226,7 +234,12 @@ __global__ void __launch_bounds__(W *Split<N>::N1)
         }
         dft_reg<T, N2, DIR>(v);
 #pragma unroll
-        for (int k1 = 1; k1 < N2; k1++) v[k1] = cmul(v[k1], tw1[k1]);
+        for (int k1 = 1; k1 < N2; k1++) {
+            if constexpr (kTwReg)
+                v[k1] = cmul(v[k1], tw1[k1]);
+            else
+                v[k1] = cmul(v[k1], twiddle(k1));
+        }
 #pragma unroll
         for (int k1 = 0; k1 < N2; k1++) B[(g + N1 * k1) * W + c] = v[k1];
         __syncthreads();

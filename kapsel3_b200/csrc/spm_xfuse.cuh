@@ -176,7 +176,7 @@ constexpr size_t x_fuse_smem() {
 }
 
 template <typename T, int N, int W, int OP, bool INV>
-__global__ void __launch_bounds__(W *Split<N>::N1, N == 256 ? 2 : 1)
+__global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
     x_fused_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant__ XArgs<T> A, unsigned int *err,
                    unsigned long long wait_ns, int skip_loads) {
     using M                       = XModes<N>;
@@ -226,7 +226,10 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N == 256 ? 2 : 1)
         int ct, o, run;
         decode((int)blockIdx.x + (q / ND) * (int)gridDim.x, ct, o, run);
         mbar_expect_tx(&full[q % S], tile_bytes);
-        tma_load_5d(buf + (size_t)(q % S) * N * W, &lmap, 2 * ct * W, o, 0, run, q % ND, &full[q % S]);
+        cplx<T> *dst = buf + (size_t)(q % S) * N * W;
+        tma_load_5d(dst, &lmap, 2 * ct * W, o, 0, run, q % ND, &full[q % S]);
+        if constexpr (N > 256)  // a box has at most 256 lines
+            tma_load_5d(dst + (size_t)N / 2 * W, &lmap, 2 * ct * W, o, N / 2, run, q % ND, &full[q % S]);
     };
     if (NF > 0 && tid == 0)
         for (int q = 0; q < S - 1 && q < nloads; q++) load(q);
@@ -463,14 +466,16 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N == 256 ? 2 : 1)
 // ---------------------------------------------------------------------------
 // Host side.
 // ---------------------------------------------------------------------------
-// Columns of a tile: 128 bytes of kz per line.
-template <typename T>
-constexpr int kXCols = sizeof(T) == 8 ? 8 : 16;
+// Columns of a tile: 128 bytes of kz per line, 64 at N = 512 (FP32; a thread of
+// an FP64 tile would need 22 modes of two accumulators, 176 registers, beside a
+// 32-point transform: FP64 runs of 512 points take the separate passes).
+template <typename T, int N>
+constexpr int kXCols = (sizeof(T) == 8 ? 8 : 16) / (N > 256 ? 2 : 1);
 
 template <typename T, int N, int OP, bool INV>
 cudaError_t x_fused_launch(const CUtensorMap &map, const XArgs<T> &A, int sm_count, unsigned int *err,
                            unsigned long long wait_ns, int skip, cudaStream_t st) {
-    constexpr int    W    = kXCols<T>;
+    constexpr int    W    = kXCols<T, N>;
     constexpr int    NT   = W * Split<N>::N1;
     constexpr size_t smem = x_fuse_smem<T, N, W, OP>();
     auto             kern = x_fused_kernel<T, N, W, OP, INV>;
@@ -494,8 +499,9 @@ cudaError_t x_fused_launch(const CUtensorMap &map, const XArgs<T> &A, int sm_cou
 template <typename T, int OP, bool INV>
 cudaError_t x_fused(const FFTPlan<T> &P, XArgs<T> A, int runs, int nslots, cudaStream_t st) {
     const Grid &g = A.g;
-    if (g.nx > 256 || g.field_elems_c() >> 32 || !encode_tiled_fn()) return cudaErrorNotSupported;
-    constexpr int W = kXCols<T>;
+    if (g.nx > (sizeof(T) == 8 ? 256 : 512) || g.field_elems_c() >> 32 || !encode_tiled_fn())
+        return cudaErrorNotSupported;
+    const int W     = g.nx > 256 ? kXCols<T, 512> : kXCols<T, 256>;
     A.ct_used       = (g.trn[2] + W - 1) / W;
     A.n_used        = outer_count(g.ny, g.trn[1]);
     A.ntiles        = A.ct_used * A.n_used * runs;
@@ -508,7 +514,7 @@ cudaError_t x_fused(const FFTPlan<T> &P, XArgs<T> A, int runs, int nslots, cudaS
         const uint64_t strides[4] = {(uint64_t)2 * g.hnzp * sizeof(T), (uint64_t)g.ny * 2 * g.hnzp * sizeof(T),
                                      (uint64_t)A.run_stride * sizeof(cplx<T>),
                                      (uint64_t)A.slot_stride * sizeof(cplx<T>)};
-        const uint32_t box[5]     = {(uint32_t)(2 * W), 1u, (uint32_t)g.nx, 1u, 1u};
+        const uint32_t box[5]     = {(uint32_t)(2 * W), 1u, (uint32_t)std::min(g.nx, 256), 1u, 1u};
         if (!make_map<T>(&map, A.u, dims, strides, box)) return cudaErrorNotSupported;
         skip = P.skip_loads > 0 ? 1 : 0;
         if (skip) P.skip_loads--;
@@ -517,6 +523,10 @@ cudaError_t x_fused(const FFTPlan<T> &P, XArgs<T> A, int runs, int nslots, cudaS
 #define SPM_XF(NN)     case NN: return x_fused_launch<T, NN, OP, INV>(map, A, P.sm_count, P.err, P.wait_ns, skip, st);
         SPM_XF(8) SPM_XF(16) SPM_XF(32) SPM_XF(64) SPM_XF(128) SPM_XF(256)
 #undef SPM_XF
+        case 512:
+            if constexpr (sizeof(T) == 4)
+                return x_fused_launch<T, 512, OP, INV>(map, A, P.sm_count, P.err, P.wait_ns, skip, st);
+            return cudaErrorNotSupported;
         default: return cudaErrorNotSupported;
     }
 }
