@@ -729,27 +729,27 @@ double stencil_bytes(const spm_ctx *c, int kind) {
 // X pass and k-space kernel.  Algorithmic bytes: the transformed fields' x
 // lines read and written plus zeta (and its compensation) read and written.
 template <typename T, int OP, bool INV>
-int x_fused_pass(spm_ctx *L, int slot, int ts_inc, bool &done) {
+int x_fused_pass(spm_ctx *L, int slot, int ts_inc, bool &done, bool zeta_too = false) {
     done = false;
     if (!L->use_tma) return SPM_OK;
     const Grid &g = L->g;
     XArgs<T>    A{};
     A.g = g;
-    A.z0 = L->cx<T>(Z0), A.z1 = L->cx<T>(Z1);
-    A.zl0 = OP == kXZeta ? nullptr : L->zl<T>(0), A.zl1 = OP == kXZeta ? nullptr : L->zl<T>(1);
+    if (OP != kXSole || zeta_too) A.z0 = L->cx<T>(Z0), A.z1 = L->cx<T>(Z1);
+    if (OP == kXNs || OP == kXProj) A.zl0 = L->zl<T>(0), A.zl1 = L->zl<T>(1);
     A.u  = L->cx<T>(slot);
     A.rw = L->rw;
     A.run_stride = L->fstride_c, A.slot_stride = L->slot_stride_c;
     A.ts_inc = ts_inc;
     A.nu = L->ph.nu, A.dt = L->ph.dt;
-    const int    nf   = OP == kXNs ? 5 : OP == kXProj ? 3 : 0;
+    const int    nf   = OP == kXNs ? 5 : OP == kXZeta ? 0 : 3;
     const double cols = (double)outer_count(g.ny, g.trn[1]) * g.trn[2] * L->fft_runs * sizeof(cplx<T>);
-    const double box  = box_bytes<T>(L, OP == kXZeta ? 2 : A.zl0 ? 8 : 4);
+    const double box  = box_bytes<T>(L, OP == kXSole ? (zeta_too ? 2 : 0) : OP == kXZeta ? 2 : A.zl0 ? 8 : 4);
     cudaEvent_t  pa   = prof_mark(L);
     const cudaError_t e = x_fused<T, OP, INV>(plan_of<T>(L), A, L->fft_runs, L->nslots - slot, L->st);
     if (e == cudaErrorNotSupported) return SPM_OK;
     SPM_CUDA_CHECK(e);
-    prof_done(L, pa, OP == kXZeta ? "x_zeta_u" : OP == kXNs ? "x_ns_update" : "x_project",
+    prof_done(L, pa, OP == kXZeta ? "x_zeta_u" : OP == kXNs ? "x_ns_update" : OP == kXProj ? "x_project" : "x_solenoidal",
               (nf + (INV ? 3 : 0)) * cols * g.nx + box);
     L->launches++;
     done = true;
@@ -843,6 +843,28 @@ int up_scatter(spm_ctx *c, bool clear = true) {
     return SPM_OK;
 }
 
+// Solenoidal_u of three real fields in place (truncated to the 2/3 box); with
+// zeta_too, zeta and uk_dc of the result as well (U_k2zeta_k of the retained
+// modes; a run without compensation words).
+template <typename T>
+int solenoidal_fields(spm_ctx *c, int slot, bool zeta_too = false) {
+    SPM_TRY(z_pass<T>(c, slot, 3, true, 1 << 30, c->g.kz_span()));
+    SPM_TRY((fft_strided_pass<T, -1>(c, slot, 3, 1, prune_forward(c->g, 1))));
+    bool done;
+    SPM_TRY((x_fused_pass<T, kXSole, true>(c, slot, 0, done, zeta_too)));
+    if (!done) {
+        SPM_TRY((fft_strided_pass<T, -1>(c, slot, 3, 0, prune_forward(c->g, 0))));
+        LAUNCH(c, k_truncate_project<T>, c->grid_blocks(), 256, 0, c->g, c->cx<T>(slot), c->cx<T>(slot + 1),
+               c->cx<T>(slot + 2), 1);
+        if (zeta_too)
+            LAUNCH(c, k_u_to_zeta<T>, c->grid_blocks(), 256, 0, c->g, c->cx<T>(slot), c->cx<T>(slot + 1),
+                   c->cx<T>(slot + 2), c->cx<T>(Z0), c->cx<T>(Z1), c->uk_dc);
+        SPM_TRY((fft_strided_pass<T, +1>(c, slot, 3, 0, prune_inverse(c->g, 0))));
+    }
+    SPM_TRY((fft_strided_pass<T, +1>(c, slot, 3, 1, prune_inverse(c->g, 1))));
+    return z_pass<T>(c, slot, 3, false, c->g.trn[2]);
+}
+
 // The self-consistent slip iteration of squirmers (the SW_JANUS_SLIP branch
 // of Time_evolution_hydro, sp_3d_ns.cxx:121-161), after the hydrodynamic
 // force: the particle and surface moments, then until convergence the slip
@@ -863,10 +885,7 @@ int slip_loop(spm_ctx *c) {
         LAUNCH(c, p_slip_droplet, pb, 128, 0, c->ph, c->slip);
         LAUNCH(c, s_slip_scatter<T>, sgrid, 128, 0, c->g, c->ph, c->ps.x, c->ps.q, c->cells, c->ncells, c->slip,
                c->real<T>(U0), c->real<T>(U1), c->real<T>(U2), c->real<T>(UP0), c->real<T>(UP1), c->real<T>(UP2));
-        SPM_TRY(fft_fwd_box<T>(c, UP0, 3));
-        LAUNCH(c, k_truncate_project<T>, c->grid_blocks(), 256, 0, c->g, c->cx<T>(UP0), c->cx<T>(UP1), c->cx<T>(UP2),
-               1);
-        SPM_TRY(fft_inv_box<T>(c, UP0, 3));
+        SPM_TRY(solenoidal_fields<T>(c, UP0));
         LAUNCH(c, s_slip_force<T>, c->ph.np, 256, 0, c->g, c->ph, c->ps.x, c->cells, c->ncells, c->real<T>(UP0),
                c->real<T>(UP1), c->real<T>(UP2), c->slip);
         LAUNCH(c, p_velocity_slip, pb, 128, 0, c->ph, c->ps, c->slip, c->ts_dev, 0);

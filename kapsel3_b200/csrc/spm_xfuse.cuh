@@ -12,6 +12,8 @@
 //           (U2advection_k's k part, NS_solver_slavedEuler)
 //   kXProj  forward X of the rigidity force f -> zeta += zeta(i k x P f)
 //           (Solenoidal_u closed in k space)
+//   kXSole  forward X of three fields -> 2/3 truncation and P -> inverse X
+//           (Solenoidal_u) [, zeta and uk_dc of the result: U_k2zeta_k]
 // The update is linear in the products, so a thread adds each product's share
 // to two accumulators per retained mode as its transform ends, and never holds
 // more than one of the five; the projection keeps the three components of f.
@@ -32,7 +34,7 @@ template <int I>
 struct XInt {
     static constexpr int value = I;
 };
-enum XOp { kXZeta = 0, kXNs = 1, kXProj = 2 };
+enum XOp { kXZeta = 0, kXNs = 1, kXProj = 2, kXSole = 3 };
 
 // Arguments of the fused passes.  Fields of run r start r * run_stride complex
 // values after run 0's; slots (fields) of a run lie slot_stride apart.
@@ -181,7 +183,8 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
                    unsigned long long wait_ns, int skip_loads) {
     using M                       = XModes<N>;
     constexpr int      N1 = M::N1, N2 = M::N2;
-    constexpr int      NF         = OP == kXNs ? 5 : OP == kXProj ? 3 : 0;
+    constexpr bool     kThree     = OP == kXProj || OP == kXSole;  // three fields, all kept
+    constexpr int      NF         = OP == kXNs ? 5 : kThree ? 3 : 0;
     constexpr int      ND         = NF > 0 ? NF : 1;  // divisor of the load sequence
     constexpr int      S          = OP == kXZeta ? 1 : kXRing;
     constexpr unsigned tile_bytes = (unsigned)(N * W * sizeof(cplx<T>));
@@ -252,15 +255,15 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
         const bool   kx0 = g == 0, ky0 = o == 0;  // at m = 0 only
         const bool   dc  = kx0 && ky0 && kz == 0;
         auto         keep = [&](int m) { return col && (M::always(m) || abs(signed_mode(g + N1 * m, N)) < M::TRN); };
-        // kXNs: the two accumulators; kXProj: the three transformed components;
-        // then zeta of the retained modes in a0, a1
-        cplx<T> a0[N2], a1[N2], a2[OP == kXProj ? N2 : 1];
+        // kXNs: the two accumulators; kXProj, kXSole: the three transformed
+        // components; then zeta of the retained modes in a0, a1 (kXSole: P f)
+        cplx<T> a0[N2], a1[N2], a2[kThree ? N2 : 1];
         if constexpr (NF > 0) {
             // zeta is needed once the fields are transformed: start it towards L2
 #pragma unroll
             for (int m = 0; m < N2; m++) {
                 a0[m] = a1[m] = cplx<T>{0, 0};
-                if (!M::maybe(m) || !keep(m)) continue;
+                if (OP == kXSole || !M::maybe(m) || !keep(m)) continue;
                 const unsigned idx = (unsigned)(g + N1 * m) * nst + line;
                 prefetch_l2(pz0 + idx);
                 prefetch_l2(pz1 + idx);
@@ -324,7 +327,8 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
                         return;
                     }
                     // the k = 0 mode takes Re f_hat(0), not touched by the projection
-                    if (dc) A.rw[run].uk_dc[f] += (double)v[0].re;
+                    if (OP == kXProj && dc) A.rw[run].uk_dc[f] += (double)v[0].re;
+                    if (OP == kXSole && dc && A.z0) A.rw[run].uk_dc[f] = (double)v[0].re;
 #pragma unroll
                     for (int m = 0; m < N2; m++) to[m] = v[m];
                 };
@@ -333,6 +337,33 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
                 take(a2, 2);
             }
             if (stopped) break;
+        }
+        if constexpr (OP == kXSole) {
+            const double dkyz2 = dky * dky + dkz * dkz;
+#pragma unroll
+            for (int m = 0; m < N2; m++) {
+                if (!M::maybe(m)) continue;
+                const double dkx = skx[g + N1 * m];
+                const T      kx  = skt[g + N1 * m], ik2 = (T)x_reciprocal<T>(dkx * dkx + dkyz2);
+                const T      dr = ik2 * (a0[m].re * kx + a1[m].re * kyt + a2[m].re * kzt);
+                const T      di = ik2 * (a0[m].im * kx + a1[m].im * kyt + a2[m].im * kzt);
+                const bool   k  = keep(m);
+                a0[m] = k ? cplx<T>{a0[m].re - dr * kx, a0[m].im - di * kx} : cplx<T>{0, 0};
+                a1[m] = k ? cplx<T>{a1[m].re - dr * kyt, a1[m].im - di * kyt} : cplx<T>{0, 0};
+                a2[m] = k ? cplx<T>{a2[m].re - dr * kzt, a2[m].im - di * kzt} : cplx<T>{0, 0};
+                if (!k || !A.z0) continue;
+                const cplx<T> u[3] = {a0[m], a1[m], a2[m]};
+                cplx<T>       om[3], z0, z1;
+                i_cross<T>(kx, kyt, kzt, u, om);
+                z0 = om[1], z1 = om[2];
+                if (m == 0 && kx0) {
+                    z0 = ky0 ? om[0] : om[2];
+                    z1 = ky0 ? om[1] : om[0];
+                }
+                const unsigned idx = (unsigned)(g + N1 * m) * nst + line;
+                pz0[idx] = z0;
+                pz1[idx] = z1;
+            }
         }
         // k-space stage: a0, a1 become zeta, ik2t 1 / k^2 for INV.  zeta of
         // kXChunk modes at a time is loaded without branches (modes outside the
@@ -344,10 +375,10 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
         const double inu   = 1.0 / A.nu;
         // 1 / k^2 for INV: kept by FP64, whose division is long; FP32 forms it again
         // for each component (seven instructions), 12 values more per thread spill
-        constexpr bool kKeepIk2 = INV && sizeof(T) == 8;
+        constexpr bool kKeepIk2 = INV && sizeof(T) == 8 && OP != kXSole;
         T              ik2t[kKeepIk2 ? N2 : 1];
 #pragma unroll
-        for (int mc = 0; mc < N2; mc += kXChunk) {
+        for (int mc = 0; OP != kXSole && mc < N2; mc += kXChunk) {
             cplx<T> z0[kXChunk], z1[kXChunk], l0[kXChunk], l1[kXChunk];
 #pragma unroll
             for (int j = 0; j < kXChunk; j++) {
@@ -364,7 +395,7 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
                 const double dkx   = skx[g + N1 * m];
                 const double k2sum = dkx * dkx + dkyz2;
                 const double ik2   = x_reciprocal<T>(k2sum);
-                if constexpr (OP != kXZeta) {
+                if constexpr (OP == kXNs || OP == kXProj) {
                     cplx<T> d0 = a0[m], d1 = a1[m];
                     if constexpr (OP == kXNs) {
                         // zeta += (e^{-nu dt k^2} - 1) (zeta - f / (nu k^2)); compensated: the
@@ -427,6 +458,10 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
                     for (int m = 0; m < N2; m++) {
                         v[m] = cplx<T>{0, 0};
                         if (!M::maybe(m)) continue;
+                        if constexpr (OP == kXSole) {
+                            v[m] = D.value == 0 ? a0[m] : D.value == 1 ? a1[m] : a2[kThree ? m : 0];
+                            continue;
+                        }
                         const T kx = skt[g + N1 * m], ikx = sik[g + N1 * m];
                         T       ik2;
                         if constexpr (kKeepIk2)
@@ -445,7 +480,7 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
                     vel(XInt<1>{});
                 else
                     vel(XInt<2>{});
-                if (dc) v[0].re = (T)A.rw[run].uk_dc[d];
+                if (OP != kXSole && dc) v[0].re = (T)A.rw[run].uk_dc[d];
                 __syncthreads();
                 x_step1<T, N, W, +1>(v, g, c, B, stw);
                 __syncthreads();
