@@ -75,18 +75,22 @@ struct FFTPlan {
 
     cudaError_t create(const Grid &grid) {
         g = grid;
-        cudaError_t e;
-        if ((e = make_table(&tw_x, g.nx, g.nx)) != cudaSuccess) return e;
-        if ((e = make_table(&tw_y, g.ny, g.ny)) != cudaSuccess) return e;
-        if ((e = make_table(&tw_zm, g.nz / 2, g.nz / 2)) != cudaSuccess) return e;
-        if ((e = make_table(&tw_zn, g.nz, g.nz / 2 + 1)) != cudaSuccess) return e;
+        // the four tables in one block and one copy
+        std::vector<cplx<T>> h;
+        add_table(h, g.nx, g.nx);
+        add_table(h, g.ny, g.ny);
+        add_table(h, g.nz / 2, g.nz / 2);
+        add_table(h, g.nz, g.nz / 2 + 1);
+        cudaError_t e = dev_alloc((void **)&tw_x, sizeof(cplx<T>) * h.size());
+        if (e != cudaSuccess) return e;
+        tw_y  = tw_x + g.nx;
+        tw_zm = tw_y + g.ny;
+        tw_zn = tw_zm + g.nz / 2;
+        if ((e = cudaMemcpy(tw_x, h.data(), sizeof(cplx<T>) * h.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return e;
         return set_smem_attrs();
     }
     void destroy() {
         dev_free(tw_x);
-        dev_free(tw_y);
-        dev_free(tw_zm);
-        dev_free(tw_zn);
         tw_x = tw_y = tw_zm = tw_zn = nullptr;
     }
 
@@ -238,15 +242,11 @@ struct FFTPlan {
     static cudaError_t configure_kernels() { return set_smem_attrs(); }
 
   private:
-    static cudaError_t make_table(cplx<T> **dst, int n, int count) {
-        std::vector<cplx<T>> h(count);
+    static void add_table(std::vector<cplx<T>> &h, int n, int count) {
         for (int j = 0; j < count; j++) {
             const long double a = -2.0L * 3.141592653589793238462643383279502884L * (long double)j / (long double)n;
-            h[j] = cplx<T>{(T)std::cos(a), (T)std::sin(a)};
+            h.push_back(cplx<T>{(T)std::cos(a), (T)std::sin(a)});
         }
-        cudaError_t e = dev_alloc((void **)dst, sizeof(cplx<T>) * count);
-        if (e != cudaSuccess) return e;
-        return cudaMemcpy(*dst, h.data(), sizeof(cplx<T>) * count, cudaMemcpyHostToDevice);
     }
     template <int NN, int DIR>
     static cudaError_t attr_one() {
