@@ -886,8 +886,8 @@ int slip_loop(spm_ctx *c) {
         LAUNCH(c, s_slip_scatter<T>, sgrid, 128, 0, c->g, c->ph, c->ps.x, c->ps.q, c->cells, c->ncells, c->slip,
                c->real<T>(U0), c->real<T>(U1), c->real<T>(U2), c->real<T>(UP0), c->real<T>(UP1), c->real<T>(UP2));
         SPM_TRY(solenoidal_fields<T>(c, UP0));
-        LAUNCH(c, s_slip_force<T>, c->ph.np, 256, 0, c->g, c->ph, c->ps.x, c->cells, c->ncells, c->real<T>(UP0),
-               c->real<T>(UP1), c->real<T>(UP2), c->slip);
+        LAUNCH(c, s_slip_force<T>, c->ph.np, 256, 0, c->g, c->ph, c->ps.x, c->cells, c->ncells, c->sc_idx, c->sc_w,
+               c->real<T>(UP0), c->real<T>(UP1), c->real<T>(UP2), c->slip);
         LAUNCH(c, p_velocity_slip, pb, 128, 0, c->ph, c->ps, c->slip, c->ts_dev, 0);
         iter++;
         LAUNCH(c, k_slip_converge, 1, 256, 0, c->ph, c->ps, c->slip, c->slip_eps);
