@@ -200,6 +200,7 @@ struct spm_ctx {
     double *     rec_stage = nullptr;  // particle records in transit (SPM_PARTICLE_WORDS per particle)
     PState       ps{};
     unsigned int *mt  = nullptr;  // 625 words
+    double       *noise = nullptr;  // thermostat: the step's six normals per particle (lone runs)
     unsigned int *err = nullptr;  // device error word (&rw->err)
     int          ts   = 0;
     double       time = 0.0;
@@ -1020,6 +1021,7 @@ PRun<T> prun_of(spm_ctx *c) {
         R.lj_bins    = R.lj_cell_of + c->ph.np;
     }
     if (c->rigid()) R.rid = c->rg.rid, R.f_lo = c->rg.f_lo;
+    R.kick = R.vel && R.noise ? c->noise : nullptr;
     R.ts = c->ts_dev, R.mt = c->mt, R.err = c->err;
     return R;
 }
@@ -1135,6 +1137,9 @@ int step_ns_runs(spm_ctx *L, spm_ctx *const *R, int nr) {
                 PLAUNCH(c, "s_phi_scatter_cache", stencil_bytes<T>(c, 0), (s_phi_scatter_cache<T, false>), sgrid, 128,
                         0, c->g, one, (const PRun<T> *)nullptr);
                 SPM_TRY(lj_forces(c, c->ph, c->rigid()));
+                // the step's normals depend on the generator alone: drawn here, added
+                // with the velocity update (s_hydro_force_cached)
+                if (one.kick) LAUNCH(c, p_thermostat, 1, kThermoThreads, 0, c->ph, c->ps, c->mt, one.kick);
                 return SPM_OK;
             };
             rc = side_work();
@@ -1168,7 +1173,7 @@ int step_ns_runs(spm_ctx *L, spm_ctx *const *R, int nr) {
         } else if (c->ph.janus_prop == SPM_JANUS_SQUIRMER) {
             SPM_TRY(slip_loop<T>(c));  // lone runs only; leaves the slip field in UP
         }
-        if (one.noise) {
+        if (one.noise && !one.kick) {
             LAUNCH(c, p_thermostat, 1, kThermoThreads, 0, c->ph, c->ps, c->mt, c->rigid() ? c->rg.noise : nullptr);
             if (c->rigid()) LAUNCH(c, r_thermostat, c->rg.nb, 128, 0, c->ph, c->ps, c->rg, c->rfree);
         }
@@ -1478,6 +1483,7 @@ void destroy_ctx(spm_ctx *c) {
     dev_free(c->pbuf);
     dev_free(c->rec_stage);
     dev_free(c->mt);
+    dev_free(c->noise);
     dev_free(c->le.dev);
     dev_free(c->le.ppart);
     dev_free(c->le.partial);
@@ -1598,7 +1604,9 @@ int create_ctx(const spm_params &p, cudaStream_t stream, int pool_cap, spm_ctx *
         dev_alloc((void **)&c->rec_stage, (size_t)std::max(np, 1) * SPM_PARTICLE_WORDS * sizeof(double)) != cudaSuccess ||
         dev_alloc((void **)&c->mt, 625 * sizeof(unsigned int)) != cudaSuccess ||
         (lj_cell_list_applies(c->ph) &&
-         dev_alloc((void **)&c->lj_list, ((size_t)lj_ncell(c->ph) * (1 + kLjBin) + np) * sizeof(int)) != cudaSuccess)) {
+         dev_alloc((void **)&c->lj_list, ((size_t)lj_ncell(c->ph) * (1 + kLjBin) + np) * sizeof(int)) != cudaSuccess) ||
+        (!lead && p.kbt > 0.0 && p.n_particles > 0 &&
+         dev_alloc((void **)&c->noise, (size_t)np * 6 * sizeof(double)) != cudaSuccess)) {
         destroy_ctx(c);
         return fail(SPM_ERR_NOMEM, "small device buffers");
     }

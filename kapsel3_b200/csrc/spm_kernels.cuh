@@ -869,6 +869,7 @@ struct PRun {
     int           ncells;
     int           vel;     // s_hydro_force_cached also updates the velocities
     int           noise;   // thermostat on
+    double       *kick;    // the step's normals, added after the velocity update, or null
     T            *phi_sum, *u0, *u1, *u2, *f0, *f1, *f2;
     int          *sc_idx;  // stencil cache
     double       *sc_w;
@@ -1008,6 +1009,13 @@ __global__ void s_hydro_force_cached(Grid g, const __grid_constant__ PRun<T> one
         // the velocities need nothing but this particle's own forces: updating
         // them here is one launch (6 to 7 us of latency on B200) fewer
         if (R.vel) velocity_update_comp(ph, s, p, d, *R.ts == 0);
+        // Add_random_force_thermostat with normals drawn beside the fluid solve: the
+        // generator's serial chain (14 us for 200 particles) leaves the main stream
+        if (R.kick) {
+            const int sp = spec_of(ph, p);
+            s.v[3 * p + d] += R.kick[6 * p + d] * ph.noise_v * ph.imass_s[sp];
+            if (ph.rotation) s.omega[3 * p + d] += R.kick[6 * p + 3 + d] * ph.noise_o * ph.imoi_s[sp];
+        }
     }
 }
 
@@ -1484,8 +1492,8 @@ __device__ __forceinline__ unsigned int mt_twist_word(const unsigned int *mt, in
     if (y & 1u) v ^= 0x9908b0dfu;
     return v;
 }
-// noise != null (rigid bodies): the six normals of particle n go to
-// noise[6 n ..], nothing is applied (r_thermostat applies them per body).
+// noise != null: the six normals of particle n go to noise[6 n ..], nothing is
+// applied (r_thermostat applies them per body, s_hydro_force_cached per sphere).
 __device__ __forceinline__ void thermostat_run(const Phys &ph, const PState &s, unsigned int *mt_g, double *noise) {
     __shared__ unsigned int mt[624];
     __shared__ double       uni[624 + 1];  // the carried uniform, then this round's outputs
