@@ -395,10 +395,9 @@ int spm_kernel_launches(spm_ctx *ctx, long long *count, int reset);
 
 /* ---- serving pool (no reference counterpart) ----------------------------
  * A pool holds independent Navier_Stokes runs of one grid size, DX and
- * precision.  Their fields share one slot-major device arena so each FFT
- * stage and each k-space pointwise kernel of a pool step is one launch over
- * all runs; particle kernels run per run on the pool's stream.  The pool step
- * can be replayed from a CUDA graph captured once per membership.  A run of
+ * precision.  Their fields share one slot-major device arena, and the runs'
+ * particle buffers are listed in a device array, so every kernel of a pool
+ * step is one launch over all runs.  The pool step can be replayed from a CUDA graph captured once per membership.  A run of
  * a pool is an spm_ctx: the whole-run getters above work on it (between
  * steps); spm_destroy refuses it (use spm_pool_release).  Releasing a run
  * moves the pool's last run into its slot; run handles stay valid. */

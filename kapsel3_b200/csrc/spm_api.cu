@@ -721,9 +721,9 @@ double stencil_bytes(const spm_ctx *c, int kind) {
 
 // ---------------------------------------------------------------------------
 // Building blocks of the step (templated on the field type).  The `_runs`
-// forms advance runs R[0..nr) that share one grid: per-run kernels go to each
-// run, FFT stages to L, which is either the run itself or a pool lead whose
-// FFT launches cover the same slots of every run of the pool.
+// forms advance runs R[0..nr) that share one grid; grid stages go to L, which
+// is either the run itself or a pool lead whose launches cover the same slots
+// of every run of the pool.
 // ---------------------------------------------------------------------------
 // One fused X pass over slots `slot`.. of every run of L (spm_xfuse.cuh).
 // Returns false where it does not apply; the caller then launches the separate
@@ -880,28 +880,24 @@ int slip_loop(spm_ctx *c) {
     const dim3 sgrid((c->ncells + 127) / 128, c->ph.np);
     LAUNCH(c, s_slip_moments<T>, c->ph.np, 256, 0, c->g, c->ph, c->ps.x, c->ps.q, c->cells, c->ncells,
            c->real<T>(U0), c->real<T>(U1), c->real<T>(U2), c->slip);
-    LAUNCH(c, p_slip_relax, pb, 128, 0, c->ph, c->ps, c->slip, 0);
     for (int iter = 0;;) {
-        for (int d = 0; d < 3; d++) SPM_CUDA_CHECK(cudaMemsetAsync(c->real<T>(UP0 + d), 0, c->field_bytes(), c->st));
-        LAUNCH(c, p_slip_droplet, pb, 128, 0, c->ph, c->slip);
+        SPM_CUDA_CHECK(cudaMemsetAsync(c->real<T>(UP0), 0, 3 * c->field_bytes(), c->st));  // a lone run: consecutive slots
+        LAUNCH(c, p_slip_next, pb, 128, 0, c->ph, c->ps, c->slip, iter);
         LAUNCH(c, s_slip_scatter<T>, sgrid, 128, 0, c->g, c->ph, c->ps.x, c->ps.q, c->cells, c->ncells, c->slip,
                c->real<T>(U0), c->real<T>(U1), c->real<T>(U2), c->real<T>(UP0), c->real<T>(UP1), c->real<T>(UP2));
         SPM_TRY(solenoidal_fields<T>(c, UP0));
         LAUNCH(c, s_slip_force<T>, c->ph.np, 256, 0, c->g, c->ph, c->ps.x, c->cells, c->ncells, c->sc_idx, c->sc_w,
-               c->real<T>(UP0), c->real<T>(UP1), c->real<T>(UP2), c->slip);
-        LAUNCH(c, p_velocity_slip, pb, 128, 0, c->ph, c->ps, c->slip, c->ts_dev, 0);
+               c->real<T>(UP0), c->real<T>(UP1), c->real<T>(UP2), c->slip, c->ps, c->ts_dev);
         iter++;
         LAUNCH(c, k_slip_converge, 1, 256, 0, c->ph, c->ps, c->slip, c->slip_eps);
         double eps = 0.0;
         SPM_CUDA_CHECK(cudaMemcpyAsync(&eps, c->slip_eps, sizeof(double), cudaMemcpyDeviceToHost, c->st));
         SPM_CUDA_CHECK(cudaStreamSynchronize(c->st));
         if (eps < c->P.slip_tol || iter == c->P.slip_iter) {
-            LAUNCH(c, p_velocity_slip, pb, 128, 0, c->ph, c->ps, c->slip, c->ts_dev, 2);
+            LAUNCH(c, p_slip_end, pb, 128, 0, c->ph, c->ps, c->slip);
             c->slip_iters = iter;
             break;
         }
-        LAUNCH(c, p_slip_relax, pb, 128, 0, c->ph, c->ps, c->slip, iter);
-        LAUNCH(c, p_velocity_slip, pb, 128, 0, c->ph, c->ps, c->slip, c->ts_dev, 1);
     }
     LAUNCH(c, r_add3<T>, c->grid_blocks(), 256, 0, c->g, c->real<T>(U0), c->real<T>(U1), c->real<T>(U2),
            c->real<T>(UP0), c->real<T>(UP1), c->real<T>(UP2));
@@ -1099,8 +1095,8 @@ int pool_main_work(spm_ctx *L, spm_ctx *const *R, int nr) {
 
 // Time_evolution_hydro (sp_3d_ns.cxx:41-194), Navier_Stokes with free
 // spheres.  L batches the grid stages of runs R[0..nr), which are L's runs in
-// order (L is the run itself for a single context); particle kernels go to
-// each run on the shared stream.
+// order (L is the run itself for a single context); a pool's particle kernels
+// are one launch over its runs (pool_side_work, pool_main_work).
 template <typename T>
 int step_ns_runs(spm_ctx *L, spm_ctx *const *R, int nr) {
     int rc;

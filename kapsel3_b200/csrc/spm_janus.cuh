@@ -179,12 +179,9 @@ __global__ void __launch_bounds__(256) s_slip_moments(Grid g, Phys ph, const dou
 // slip_droplet (operate_surface.cxx:155-195): the velocity delta_v, delta_w
 // of the counter-flow inside the particle that keeps the momentum change of
 // the enforced slip (taken w.r.t. v_slip, omega_slip) at zero.  The 3 x 3
-// inverse is the cofactor form of M_inv (lad3.h:219-236).  Thread per
-// particle.
-__global__ void p_slip_droplet(Phys ph, double *__restrict__ slip) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= ph.np || ph.janus_prop != 2) return;
-    double      *sp = slip + (size_t)n * kSlipWords;
+// inverse is the cofactor form of M_inv (lad3.h:219-236).
+__device__ __forceinline__ void slip_droplet_one(const Phys &ph, double *sp) {
+    if (ph.janus_prop != 2) return;
     const double *vp = sp + kSlipV, *wp = sp + kSlipW, *mc = sp + kSlipMC, *smc = sp + kSlipSMC;
     const double *I = sp + kSlipI, *SI = sp + kSlipSI;
     const double imass = 1.0 / sp[kSlipMass];
@@ -282,6 +279,32 @@ __global__ void s_slip_scatter(Grid g, Phys ph, const double *__restrict__ x, co
     }
 }
 
+// MD_solver_velocity_slip_iter (particle_solver.cxx:209-237, start / new)
+// without its Force() call (the step computes the LJ and body forces
+// beforehand): component d of the Euler or AB2 update with f_hydro + f_slip
+// (slip Euler / AB2, particle_solver.cxx:144-207).
+__device__ __forceinline__ void velocity_slip_comp(const Phys &ph, const PState &s, const double *sp, int n, int d,
+                                                   int euler) {
+    const double dmy = (euler ? ph.dt : ph.hdt) * ph.imass_s[spec_of(ph, n)];
+    const double dmr = (euler ? ph.dt : ph.hdt) * ph.imoi_s[spec_of(ph, n)];
+    double       sf[3], st[3];
+    self_propulsion_d(ph, s.q + 4 * n, sf, st);
+    const double sfd = d == 0 ? sf[0] : d == 1 ? sf[1] : sf[2];
+    const double std = d == 0 ? st[0] : d == 1 ? st[1] : st[2];
+    const int    i   = 3 * n + d;
+    s.v_old[i]       = s.v[i];
+    s.omega_old[i]   = s.omega[i];
+    if (ph.janus_prop == 3) {
+        s.v[i] = 0.0, s.omega[i] = 0.0;
+    } else if (euler) {
+        s.v[i] += dmy * (s.f_hydro[i] + sp[kSlipF + d] + s.fr[i] + sfd);
+        s.omega[i] += dmr * (s.torque_hydro[i] + sp[kSlipT + d] + s.torque_r[i] + std);
+    } else {
+        s.v[i] += dmy * (2.0 * (s.f_hydro[i] + sp[kSlipF + d] + sfd) + s.fr[i] + s.fr_previous[i]);
+        s.omega[i] += dmr * (2.0 * (s.torque_hydro[i] + sp[kSlipT + d] + std) + s.torque_r[i] + s.torque_r_previous[i]);
+    }
+}
+
 // Calc_f_slip_correct_precision (md_force.cxx:325-382): f_slip = DX^3 RHO /
 // dt sum phi up, torque_slip = DX^3 RHO / dt sum r x (phi up).  One CTA per
 // particle, index and profile of its cells from the step's stencil cache and the
@@ -293,7 +316,8 @@ __global__ void __launch_bounds__(256) s_slip_force(Grid g, Phys ph, const doubl
                                                     const int *__restrict__ cells, int ncells,
                                                     const int *__restrict__ sc_idx, const double *__restrict__ sc_w,
                                                     const T *__restrict__ up0, const T *__restrict__ up1,
-                                                    const T *__restrict__ up2, double *__restrict__ slip) {
+                                                    const T *__restrict__ up2, double *__restrict__ slip, PState s,
+                                                    const int *__restrict__ ts_dev) {
     const int p = blockIdx.x;
     if (p >= ph.np) return;
     const double xp[3] = {x[3 * p], x[3 * p + 1], x[3 * p + 2]};
@@ -335,86 +359,64 @@ __global__ void __launch_bounds__(256) s_slip_force(Grid g, Phys ph, const doubl
         }
     }
     block_sum6(acc);
-    if (threadIdx.x == 0) {
+    // component d by lane d of the first warp, which holds the sums; the velocity
+    // update needs this particle's force alone
+    if (threadIdx.x < 3) {
+        const int    d   = threadIdx.x;
         const double dmy = ph.dx3 * ph.rho / ph.dt;
         double      *sp  = slip + (size_t)p * kSlipWords;
-        for (int d = 0; d < 6; d++) sp[kSlipF + d] = dmy * acc[d];
+        sp[kSlipF + d]   = dmy * (d == 0 ? acc[0] : d == 1 ? acc[1] : acc[2]);
+        sp[kSlipT + d]   = dmy * (d == 0 ? acc[3] : d == 1 ? acc[4] : acc[5]);
+        velocity_slip_comp(ph, s, sp, p, d, *ts_dev == 0);
     }
 }
 
-// MD_solver_velocity_slip_iter (particle_solver.cxx:209-237) without its
-// Force() call (the step computes the LJ and body forces beforehand).
-// mode 0 (start / new): the Euler or AB2 update with f_hydro + f_slip (slip
-// Euler / AB2, particle_solver.cxx:144-207); 1 (reset): v, omega back to
-// v_old, omega_old; 2 (end): reset_Forces (particle_solver.cxx:11-37).
-__global__ void p_velocity_slip(Phys ph, PState s, double *__restrict__ slip, const int *__restrict__ ts_dev,
-                                int mode) {
+// reset_Forces (particle_solver.cxx:11-37) at the end of the slip iteration.
+__global__ void p_slip_end(Phys ph, PState s, double *__restrict__ slip) {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= ph.np) return;
     double *sp = slip + (size_t)n * kSlipWords;
-    if (mode == 0) {
-        const int    euler = *ts_dev == 0;
-        const double dmy   = (euler ? ph.dt : ph.hdt) * ph.imass_s[spec_of(ph, n)];
-        const double dmr   = (euler ? ph.dt : ph.hdt) * ph.imoi_s[spec_of(ph, n)];
-        double       sf[3], st[3];
-        self_propulsion_d(ph, s.q + 4 * n, sf, st);
-        for (int d = 0; d < 3; d++) {
-            const int i    = 3 * n + d;
-            s.v_old[i]     = s.v[i];
-            s.omega_old[i] = s.omega[i];
-            if (ph.janus_prop == 3) {
-                s.v[i] = 0.0, s.omega[i] = 0.0;
-            } else if (euler) {
-                s.v[i] += dmy * (s.f_hydro[i] + sp[kSlipF + d] + s.fr[i] + sf[d]);
-                s.omega[i] += dmr * (s.torque_hydro[i] + sp[kSlipT + d] + s.torque_r[i] + st[d]);
-            } else {
-                s.v[i] += dmy * (2.0 * (s.f_hydro[i] + sp[kSlipF + d] + sf[d]) + s.fr[i] + s.fr_previous[i]);
-                s.omega[i] += dmr * (2.0 * (s.torque_hydro[i] + sp[kSlipT + d] + st[d]) + s.torque_r[i] +
-                                     s.torque_r_previous[i]);
-            }
-        }
-    } else if (mode == 1) {
-        for (int d = 0; d < 3; d++) {
-            const int i = 3 * n + d;
-            s.v[i]      = s.v_old[i];
-            s.omega[i]  = s.omega_old[i];
-        }
-    } else {
-        for (int d = 0; d < 3; d++) {
-            const int i                = 3 * n + d;
-            s.fr_previous[i]           = s.fr[i];
-            s.fr[i]                    = 0.0;
-            s.f_hydro_previous[i]      = s.f_hydro[i];
-            s.f_hydro[i]               = 0.0;
-            sp[kSlipFPrev + d]         = sp[kSlipF + d];
-            sp[kSlipF + d]             = 0.0;
-            s.torque_r_previous[i]     = s.torque_r[i];
-            s.torque_r[i]              = 0.0;
-            s.torque_hydro_previous[i] = s.torque_hydro[i];
-            s.torque_hydro[i]          = 0.0;
-            sp[kSlipTPrev + d]         = sp[kSlipT + d];
-            sp[kSlipT + d]             = 0.0;
-        }
+    for (int d = 0; d < 3; d++) {
+        const int i                = 3 * n + d;
+        s.fr_previous[i]           = s.fr[i];
+        s.fr[i]                    = 0.0;
+        s.f_hydro_previous[i]      = s.f_hydro[i];
+        s.f_hydro[i]               = 0.0;
+        sp[kSlipFPrev + d]         = sp[kSlipF + d];
+        sp[kSlipF + d]             = 0.0;
+        s.torque_r_previous[i]     = s.torque_r[i];
+        s.torque_r[i]              = 0.0;
+        s.torque_hydro_previous[i] = s.torque_hydro[i];
+        s.torque_hydro[i]          = 0.0;
+        sp[kSlipTPrev + d]         = sp[kSlipT + d];
+        sp[kSlipT + d]             = 0.0;
     }
 }
 
-// Update_slip_particle_velocity (operate_surface.h:95-116): iter 0 copies
-// v, omega; later iterations relax with weight 0.7 on the new velocity.
-__global__ void p_slip_relax(Phys ph, const PState s, double *__restrict__ slip, int iter) {
+// Start of slip iteration iter, one thread per particle: v_slip takes v, omega
+// (iter 0) or relaxes towards them with weight 0.7 (Update_slip_particle_
+// velocity, operate_surface.h:95-116), v and omega return to v_old and
+// omega_old (the reset of MD_solver_velocity_slip_iter), then the droplet's
+// counter-flow (slip_droplet).
+__global__ void p_slip_next(Phys ph, PState s, double *__restrict__ slip, int iter) {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= ph.np) return;
     double      *sp      = slip + (size_t)n * kSlipWords;
     const double dmy_new = 0.7;
     const double dmy_old = 1.0 - dmy_new;
     for (int d = 0; d < 3; d++) {
+        const int i = 3 * n + d;
         if (iter == 0) {
-            sp[kSlipV + d] = s.v[3 * n + d];
-            sp[kSlipW + d] = s.omega[3 * n + d];
+            sp[kSlipV + d] = s.v[i];
+            sp[kSlipW + d] = s.omega[i];
         } else {
-            sp[kSlipV + d] = dmy_old * sp[kSlipV + d] + dmy_new * s.v[3 * n + d];
-            sp[kSlipW + d] = dmy_old * sp[kSlipW + d] + dmy_new * s.omega[3 * n + d];
+            sp[kSlipV + d] = dmy_old * sp[kSlipV + d] + dmy_new * s.v[i];
+            sp[kSlipW + d] = dmy_old * sp[kSlipW + d] + dmy_new * s.omega[i];
+            s.v[i]         = s.v_old[i];
+            s.omega[i]     = s.omega_old[i];
         }
     }
+    slip_droplet_one(ph, sp);
 }
 
 // Slip_particle_convergence (operate_surface.h:64-94): sqrt of the largest
