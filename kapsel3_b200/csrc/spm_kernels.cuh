@@ -1075,7 +1075,7 @@ __device__ __forceinline__ void qtn_normalize_d(double *q) {
 // MD_solver_position_Euler / _AB2 (particle_solver.cxx:39-85) with the
 // orientation updates (particle_rotation_solver.h:23-29, 72-81) and PBC
 // (periodic_boundary.h:9-16).
-// wrap = 0 leaves the periodic wrap to p_le_wrap (Lees-Edwards image).
+// wrap = 0 leaves the periodic wrap to p_position_le (Lees-Edwards image).
 // The Euler start (ts == 0) is read from the run's device step counter, so a
 // captured step graph serves every step.
 __device__ __forceinline__ void position_one(const Phys &ph, const PState &s, int n, int euler, int wrap) {

@@ -416,7 +416,7 @@ __global__ void r_le_reset(Grid g, const T *__restrict__ u0, const T *__restrict
 // adds every kLeFinishThreads-th term, a tree over the block follows, so the
 // order is fixed.  One thread walking the list waits for every load in turn
 // (2368 partials: 86 us a launch on B200, 128^3 and 64^3 alike; a block of
-// 1024 takes 3 us).
+// 1024 takes 4 us).
 constexpr int kLeFinishThreads = 1024;
 
 // Shear_rate_eff = shear_rate + ivol * sum (set once per step)

@@ -1,5 +1,5 @@
-"""Block sums of the Lees-Edwards step (k_le_finish_reduction,
-k_le_stress_finish): the stress line against the oracle for particle counts
+"""Block sums of the Lees-Edwards step (k_le_shear_rate,
+k_le_step_finish): the stress line against the oracle for particle counts
 below, at and above one block of 1024 threads.
 
 FP64 sums of n terms in another order differ by at most about n 2^-53 of the
