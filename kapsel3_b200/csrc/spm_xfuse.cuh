@@ -157,16 +157,18 @@ __device__ __forceinline__ cplx<T> x_velocity(T kx, T ky, T kz, T ik2, T inv_kx,
     return cplx<T>{-(kx * om[1].im - ky * om[0].im), kx * om[1].re - ky * om[0].re};
 }
 
-// 1 / k^2 (0 at k = 0).  FP32 needs it to FP32 rounding only: one Newton step
-// in FP64 from the approximate FP32 reciprocal (1 ulp) leaves an error below
-// 2^-44.
+// 1 / k^2 (0 at k = 0) from the approximate FP32 reciprocal (1 ulp, x_fused
+// checks that k^2 is in its range): a Newton step in FP64 leaves an error below
+// 2^-44, enough for FP32; FP64 takes a second, whose last operation rounds once
+// (the error before it is below 2^-88), as a division does.
 template <typename T>
 __device__ __forceinline__ double x_reciprocal(double k2) {
-    if (sizeof(T) == 8) return k2 > 0.0 ? 1.0 / k2 : 0.0;
     float r;
     asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"((float)k2));
-    const double y = (double)r;
-    return k2 > 0.0 ? y * (2.0 - k2 * y) : 0.0;
+    double y = (double)r;
+    y        = fma(y, fma(-k2, y, 1.0), y);
+    if (sizeof(T) == 8) y = fma(y, fma(-k2, y, 1.0), y);
+    return k2 > 0.0 ? y : 0.0;
 }
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
@@ -365,7 +367,7 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
                 pz1[idx] = z1;
             }
         }
-        // k-space stage: a0, a1 become zeta, ik2t 1 / k^2 for INV.  zeta of
+        // k-space stage: a0, a1 become zeta.  zeta of
         // kXChunk modes at a time is loaded without branches (modes outside the
         // box read the run's first element), so its loads are in flight together.
         // e^{x + y} - 1 = ex + ey + ex ey for x, y <= 0 has no cancellation, so a
@@ -373,10 +375,6 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
         const double dkyz2 = dky * dky + dkz * dkz;
         const double eyz   = OP == kXNs ? expm1(-A.nu * A.dt * dkyz2) : 0.0;
         const double inu   = 1.0 / A.nu;
-        // 1 / k^2 for INV: kept by FP64, whose division is long; FP32 forms it again
-        // for each component (seven instructions), 12 values more per thread spill
-        constexpr bool kKeepIk2 = INV && sizeof(T) == 8 && OP != kXSole;
-        T              ik2t[kKeepIk2 ? N2 : 1];
 #pragma unroll
         for (int mc = 0; OP != kXSole && mc < N2; mc += kXChunk) {
             cplx<T> z0[kXChunk], z1[kXChunk], l0[kXChunk], l1[kXChunk];
@@ -437,7 +435,6 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
                 if constexpr (INV) {
                     a0[m] = keep(m) ? z0[j] : cplx<T>{0, 0};
                     a1[m] = keep(m) ? z1[j] : cplx<T>{0, 0};
-                    if constexpr (kKeepIk2) ik2t[m] = (T)ik2;
                 }
             }
         }
@@ -463,11 +460,9 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
                             continue;
                         }
                         const T kx = skt[g + N1 * m], ikx = sik[g + N1 * m];
-                        T       ik2;
-                        if constexpr (kKeepIk2)
-                            ik2 = ik2t[m];
-                        else
-                            ik2 = (T)x_reciprocal<T>(skx[g + N1 * m] * skx[g + N1 * m] + dkyz2);
+                        // formed again for each component: kept, its 12 values per thread spill
+                        // (ten steps at 256^3: FP64 15674 against 15280 us, FP32 10143 against 9929)
+                        const T ik2 = (T)x_reciprocal<T>(skx[g + N1 * m] * skx[g + N1 * m] + dkyz2);
                         if (m == 0)
                             v[m] = x_velocity<T, D.value, true>(kx, kyt, kzt, ik2, ikx, kx0, ky0, kz_ky, a0[m], a1[m]);
                         else
@@ -536,6 +531,13 @@ cudaError_t x_fused(const FFTPlan<T> &P, XArgs<T> A, int runs, int nslots, cudaS
     const Grid &g = A.g;
     if (g.nx > (sizeof(T) == 8 ? 256 : 512) || g.field_elems_c() >> 32 || !encode_tiled_fn())
         return cudaErrorNotSupported;
+    double kmin = 1e300, kmax = 0.0;  // x_reciprocal's range
+    for (int d = 0; d < 3; d++) {
+        const double n = d == 0 ? g.nx : d == 1 ? g.ny : g.nz;
+        kmin           = std::min(kmin, g.wave[d] * g.wave[d]);
+        kmax += 0.25 * n * n * g.wave[d] * g.wave[d];
+    }
+    if (!(kmin > 1e-30) || !(kmax < 1e30)) return cudaErrorNotSupported;
     const int W     = g.nx > 256 ? kXCols<T, 512> : kXCols<T, 256>;
     A.ct_used       = (g.trn[2] + W - 1) / W;
     A.n_used        = outer_count(g.ny, g.trn[1]);
