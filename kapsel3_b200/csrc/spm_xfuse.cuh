@@ -25,7 +25,7 @@
 // threads fit an SM with a three-tile TMA ring each.
 #pragma once
 
-#include "spm_fft.cuh"
+#include "spm_fft_plan.cuh"
 #include "spm_kernels.cuh"
 
 namespace spm {
@@ -60,7 +60,22 @@ struct XModes {
     static constexpr bool maybe(int m) { return N1 * m < TRN || N1 * m + N1 - 1 > N - TRN; }
     // whether it is one for every g < N1
     static constexpr bool always(int m) { return N1 * m + N1 - 1 < TRN || N1 * m > N - TRN; }
+    static __host__ __device__ __forceinline__ bool retained(int g, int m) {
+        const int k = signed_mode(g + N1 * m, N);
+        return always(m) || (k < TRN && -k < TRN);
+    }
+    // The index whose zeta the thread of n = g + N1 m loads, without a branch: n
+    // itself, or where n is outside the box its own first mode (always inside: N1
+    // <= TRN).  Nobody but this thread writes that word; one word for all such
+    // threads would be read while the thread that owns it writes it.
+    static __host__ __device__ __forceinline__ int zeta_index(int g, int m) { return retained(g, m) ? g + N1 * m : g; }
 };
+// Element offset of column kz of ky line o inside a field.  A tile reaches past
+// the retained columns; those beyond the row share its last column, which is
+// outside the box (hnz - 1 = NZ/2 >= trn), so that no thread writes it.
+__host__ __device__ __forceinline__ unsigned x_line(const Grid &g, int o, int kz) {
+    return (unsigned)o * g.hnzp + (kz < g.hnzp ? kz : g.hnzp - 1);
+}
 
 // Twiddled step 1 of the four-step transform on v[m] = x[g + N1 m], its
 // results to rows g + N1 k1 of the exchange tile B.  stw[N1 k1 + g] =
@@ -247,7 +262,7 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
         const bool   col  = kz < gr.trn[2];
         const size_t ro   = (size_t)run * A.run_stride;
         // element offsets inside a field fit 32 bits (x_fused checks it)
-        const unsigned line = (unsigned)o * gr.hnzp + kz;  // + n * nst for index n
+        const unsigned line = x_line(gr, o, kz);  // + n * nst for index n
         const unsigned nst  = (unsigned)gr.ny * gr.hnzp;
         cplx<T>  *pz0 = A.z0 + ro, *pz1 = A.z1 + ro;
         const bool comp = sizeof(T) == 4 && A.zl0 != nullptr;
@@ -256,7 +271,7 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
         const T      kyt = (T)dky, kzt = (T)dkz;
         const bool   kx0 = g == 0, ky0 = o == 0;  // at m = 0 only
         const bool   dc  = kx0 && ky0 && kz == 0;
-        auto         keep = [&](int m) { return col && (M::always(m) || abs(signed_mode(g + N1 * m, N)) < M::TRN); };
+        auto         keep = [&](int m) { return col && M::retained(g, m); };
         // kXNs: the two accumulators; kXProj, kXSole: the three transformed
         // components; then zeta of the retained modes in a0, a1 (kXSole: P f)
         cplx<T> a0[N2], a1[N2], a2[kThree ? N2 : 1];
@@ -367,9 +382,9 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
                 pz1[idx] = z1;
             }
         }
-        // k-space stage: a0, a1 become zeta.  zeta of
-        // kXChunk modes at a time is loaded without branches (modes outside the
-        // box read the run's first element), so its loads are in flight together.
+        // k-space stage: a0, a1 become zeta.  zeta of kXChunk modes at a time is
+        // loaded without branches (XModes::zeta_index), so its loads are in flight
+        // together; what a mode outside the box loads is dropped.
         // e^{x + y} - 1 = ex + ey + ex ey for x, y <= 0 has no cancellation, so a
         // mode costs no exponential of its own.
         const double dkyz2 = dky * dky + dkz * dkz;
@@ -382,7 +397,7 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
             for (int j = 0; j < kXChunk; j++) {
                 const int m = mc + j;
                 if (m >= N2 || !M::maybe(m)) continue;
-                const unsigned idx = keep(m) ? (unsigned)(g + N1 * m) * nst + line : 0u;
+                const unsigned idx = (unsigned)M::zeta_index(g, m) * nst + line;
                 z0[j] = pz0[idx], z1[j] = pz1[idx];
                 if (OP != kXZeta && comp) l0[j] = pl0[idx], l1[j] = pl1[idx];
             }
