@@ -233,7 +233,7 @@ struct spm_ctx {
     std::vector<ProfRec> prof;
     bool                     use_tma    = true;  // SPM_NO_TMA=1 selects the direct-load passes
     bool                     overlap    = true;  // SPM_NO_OVERLAP=1 keeps the particle work on the main stream
-    bool                     zeta_dirty = false;  // zeta set by the host since the last NS step
+    bool                     zeta_dirty = false;  // zeta may hold modes outside the 2/3 box (set from outside a step)
     int                      nslots     = NSLOT;  // field slots of this run (slots_for)
     AvsOut                  *avs        = nullptr;  // AVS field/particle output (spm_avs_open)
     UdfOut                  *udf_out    = nullptr;  // UDF particle records (spm_udf_out_open)
