@@ -1576,6 +1576,7 @@ int create_ctx(const spm_params &p, cudaStream_t stream, int pool_cap, spm_ctx *
             destroy_ctx(c);
             return fail(SPM_ERR_CUDA, std::string("FFT plan: ") + cudaGetErrorString(e));
         }
+        c->fp64() ? x_fused_setup(c->plan64) : x_fused_setup(c->plan32);
         if (pool_cap > 0) {
             cudaMemset(c->rw, 0, (size_t)(pool_cap + 1) * sizeof(RunWords));
             c->uk_dc  = c->rw->uk_dc;

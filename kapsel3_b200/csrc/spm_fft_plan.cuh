@@ -166,6 +166,7 @@ struct FFTPlan {
     mutable int skip_loads = 0;
     int           ctas_per_sm = 1;
     int           sm_count    = 148;
+    int           x_occ[5]    = {};  // resident CTAs per SM of the fused X passes (x_fused_setup); 0: not available
 
     template <int DIR>
     cudaError_t strided_tma(cplx<T> *data, int nfields, size_t fs_c, int nruns, size_t run_stride_c, int axis,
@@ -237,8 +238,8 @@ struct FFTPlan {
         return strided<DIR>(data, nfields, fs_c, axis, st, PassPrune::full(g.hnz));
     }
 
-    // Sets the shared-memory limits of every FFT kernel (process-wide
-    // function attributes; no allocation).
+    // Sets the shared-memory limits of every FFT kernel (function attributes
+    // of the current device; no allocation).
     static cudaError_t configure_kernels() { return set_smem_attrs(); }
 
   private:

@@ -517,30 +517,61 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
 template <typename T, int N>
 constexpr int kXCols = (sizeof(T) == 8 ? 8 : 16) / (N > 256 ? 2 : 1);
 
+// Index of an instance's occupancy in FFTPlan::x_occ.
+constexpr int x_instance(int op, bool inv) { return op == kXNs && !inv ? 4 : op; }
+
+// Raises the shared-memory limit of one instance on the current device and asks
+// how many of its CTAs an SM holds there.  Both belong to the device, so they are
+// taken at every plan creation and kept in the plan: asked once per process, a
+// context on another device would launch without its limit.  0: not available
+// (the caller takes the separate passes).
 template <typename T, int N, int OP, bool INV>
-cudaError_t x_fused_launch(const CUtensorMap &map, const XArgs<T> &A, int sm_count, unsigned int *err,
-                           unsigned long long wait_ns, int skip, cudaStream_t st) {
+int x_fused_occupancy() {
     constexpr int    W    = kXCols<T, N>;
-    constexpr int    NT   = W * Split<N>::N1;
     constexpr size_t smem = x_fuse_smem<T, N, W, OP>();
     auto             kern = x_fused_kernel<T, N, W, OP, INV>;
-    // resident CTAs per SM, asked once per instance
-    static const int occ = [&] {
-        int n = 0;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, NT, smem) != cudaSuccess)
-            n = 0;
-        return n;
-    }();
-    if (occ < 1) return cudaErrorNotSupported;
-    const int grid = std::min(A.ntiles, sm_count * occ);
-    kern<<<grid, NT, smem, st>>>(map, A, err, wait_ns, skip);
+    int              n    = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, W * Split<N>::N1, smem) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    return n;
+}
+template <typename T, int N>
+void x_fused_setup_n(FFTPlan<T> &P) {
+    P.x_occ[x_instance(kXZeta, true)] = x_fused_occupancy<T, N, kXZeta, true>();
+    P.x_occ[x_instance(kXNs, true)]   = x_fused_occupancy<T, N, kXNs, true>();
+    P.x_occ[x_instance(kXNs, false)]  = x_fused_occupancy<T, N, kXNs, false>();
+    P.x_occ[x_instance(kXProj, true)] = x_fused_occupancy<T, N, kXProj, false>();
+    P.x_occ[x_instance(kXSole, true)] = x_fused_occupancy<T, N, kXSole, true>();
+}
+// The instances of the plan's axis, on the current device.
+template <typename T>
+void x_fused_setup(FFTPlan<T> &P) {
+    switch (P.g.nx) {
+#define SPM_XF(NN) case NN: x_fused_setup_n<T, NN>(P); break;
+        SPM_XF(8) SPM_XF(16) SPM_XF(32) SPM_XF(64) SPM_XF(128) SPM_XF(256)
+#undef SPM_XF
+        case 512:
+            if constexpr (sizeof(T) == 4) x_fused_setup_n<T, 512>(P);
+            break;
+        default: break;
+    }
+}
+
+template <typename T, int N, int OP, bool INV>
+cudaError_t x_fused_launch(const CUtensorMap &map, const XArgs<T> &A, int ctas, unsigned int *err,
+                           unsigned long long wait_ns, int skip, cudaStream_t st) {
+    constexpr int W = kXCols<T, N>;
+    x_fused_kernel<T, N, W, OP, INV><<<std::min(A.ntiles, ctas), W * Split<N>::N1, x_fuse_smem<T, N, W, OP>(), st>>>(
+        map, A, err, wait_ns, skip);
     return cudaGetLastError();
 }
 
 // One fused X pass.  Returns cudaErrorNotSupported where it cannot run (an
-// axis longer than a TMA box, no tensor-map entry point); the caller then
-// takes the separate passes.
+// FP64 axis of 512 points, no tensor-map entry point, no resident CTA); the
+// caller then takes the separate passes.
 template <typename T, int OP, bool INV>
 cudaError_t x_fused(const FFTPlan<T> &P, XArgs<T> A, int runs, int nslots, cudaStream_t st) {
     const Grid &g = A.g;
@@ -558,6 +589,8 @@ cudaError_t x_fused(const FFTPlan<T> &P, XArgs<T> A, int runs, int nslots, cudaS
     A.n_used        = outer_count(g.ny, g.trn[1]);
     A.ntiles        = A.ct_used * A.n_used * runs;
     A.tw            = P.tw_x;
+    const int ctas  = P.sm_count * P.x_occ[x_instance(OP, INV)];
+    if (ctas < 1) return cudaErrorNotSupported;
     CUtensorMap map{};
     int         skip = 0;
     if (OP != kXZeta) {
@@ -572,12 +605,12 @@ cudaError_t x_fused(const FFTPlan<T> &P, XArgs<T> A, int runs, int nslots, cudaS
         if (skip) P.skip_loads--;
     }
     switch (g.nx) {
-#define SPM_XF(NN)     case NN: return x_fused_launch<T, NN, OP, INV>(map, A, P.sm_count, P.err, P.wait_ns, skip, st);
+#define SPM_XF(NN)     case NN: return x_fused_launch<T, NN, OP, INV>(map, A, ctas, P.err, P.wait_ns, skip, st);
         SPM_XF(8) SPM_XF(16) SPM_XF(32) SPM_XF(64) SPM_XF(128) SPM_XF(256)
 #undef SPM_XF
         case 512:
             if constexpr (sizeof(T) == 4)
-                return x_fused_launch<T, 512, OP, INV>(map, A, P.sm_count, P.err, P.wait_ns, skip, st);
+                return x_fused_launch<T, 512, OP, INV>(map, A, ctas, P.err, P.wait_ns, skip, st);
             return cudaErrorNotSupported;
         default: return cudaErrorNotSupported;
     }
