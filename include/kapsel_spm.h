@@ -440,7 +440,8 @@ int spm_debug_skip_tma_loads(spm_ctx *ctx, int launches);
 /* Device memory of contexts and pools comes from a stream-ordered memory pool
  * per device that keeps freed blocks mapped for reuse, because cudaFree waits
  * for the whole device and unmaps (up to 0.8 s for a pool arena on B200).
- * This returns the unused part to the driver; bytes = what was held unused. */
+ * This returns the unused part to the driver; bytes = what was held unused.
+ * Small pinned host blocks of destroyed pools (at most 1 MB in all) go with it. */
 int spm_release_cached_memory(size_t *bytes);
 
 /* ---- serving loop (no reference counterpart) -----------------------------
