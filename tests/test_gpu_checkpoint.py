@@ -39,6 +39,10 @@ CASES = {
                                       kbt=1.0, salt=True, valency=(1.0, -1.0), onsager=(1.0, 1.5), debye_length=5.0,
                                       surface_charge=-12.0, e_field="AC", e_ext=(0.1, 0.05, 0.0), e_frequency=4.0),
                             N.SPM_PREC_FP64),
+    "electrolyte_fp32": (SPMConfig(npx=5, npy=4, npz=5, n_particles=2, a=3.0, a_xi=2.0, dt=0.01, equation=EQ_EL,
+                                   kbt=1.0, salt=True, valency=(1.0, -1.0), onsager=(1.0, 1.5), debye_length=5.0,
+                                   surface_charge=-12.0, e_field="DC", e_ext=(0.1, 0.05, 0.0)),
+                         N.SPM_PREC_FP32_MIXED),
 }
 
 
@@ -94,6 +98,22 @@ def test_checkpoint_is_refused_by_another_run(gpu, tmp_path):
     with SPMRun(cfg, precision=prec) as b:
         with pytest.raises(N.SpmError, match="truncated"):
             b.load_state(short)
+
+
+def test_electrolyte_fp32_state_without_its_ions_is_refused(gpu, tmp_path):
+    """Version 1 of an FP32 Electrolyte state does not hold the ion concentrations."""
+    cfg, prec = CASES["electrolyte_fp32"]
+    path = os.path.join(tmp_path, "el.ck")
+    with SPMRun(cfg, precision=prec) as a:
+        a.initialize(make_particles(cfg, seed=4))
+        a.step(1)
+        a.save_state(path)
+        data = bytearray(open(path, "rb").read())
+        assert int.from_bytes(data[8:12], "little") == 2
+        data[8:12] = (1).to_bytes(4, "little")
+        open(path, "wb").write(data)
+        with pytest.raises(N.SpmError, match="version"):
+            a.load_state(path)
 
 
 def test_shear_checkpoint_keeps_its_profile(gpu, tmp_path):
