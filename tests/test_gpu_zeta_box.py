@@ -61,6 +61,7 @@ def test_zeta_of_a_velocity(gpu, eq, prec, more):
         run.step(1)
         z, dc = run.U_k2zeta_k(k)
         assert z[:, ~box].any()
+        assert np.array_equal(run.zeta()[0], z)  # no compensation left of the zeta before
         run.step(2)
         got, _ = run.zeta()
     assert not got[:, ~box].any()
