@@ -784,12 +784,31 @@ double stencil_bytes(const spm_ctx *c, int kind) {
 // is either the run itself or a pool lead whose launches cover the same slots
 // of every run of the pool.
 // ---------------------------------------------------------------------------
-// One fused X pass over slots `slot`.. of every run of L (spm_xfuse.cuh).
-// Returns false where it does not apply; the caller then launches the separate
+// Consecutive runs of a pool with the same viscosity and time step, the physical
+// constants of the fluid's update: one launch of it each.
+struct RunGroup {
+    int    first, count;
+    double nu, dt;
+};
+std::vector<RunGroup> run_groups(spm_ctx *const *R, int nr) {
+    std::vector<RunGroup> out;
+    for (int r = 0; r < nr; r++) {
+        const Phys &ph = R[r]->ph;
+        if (!out.empty() && out.back().nu == ph.nu && out.back().dt == ph.dt)
+            out.back().count++;
+        else
+            out.push_back({r, 1, ph.nu, ph.dt});
+    }
+    return out;
+}
+
+// One fused X pass over slots `slot`.. of every run of L, or of the runs of
+// `group` (spm_xfuse.cuh).  Returns false where it does not apply; the caller then launches the separate
 // X pass and k-space kernel.  Algorithmic bytes: the transformed fields' x
 // lines read and written plus zeta (and its compensation) read and written.
 template <typename T, int OP, bool INV>
-int x_fused_pass(spm_ctx *L, int slot, int ts_inc, bool &done, bool zeta_too = false) {
+int x_fused_pass(spm_ctx *L, int slot, int ts_inc, bool &done, bool zeta_too = false,
+                 const RunGroup *group = nullptr) {
     done = false;
     if (!L->use_tma) return SPM_OK;
     const Grid &g = L->g;
@@ -802,11 +821,19 @@ int x_fused_pass(spm_ctx *L, int slot, int ts_inc, bool &done, bool zeta_too = f
     A.run_stride = L->fstride_c, A.slot_stride = L->slot_stride_c;
     A.ts_inc = ts_inc;
     A.nu = L->ph.nu, A.dt = L->ph.dt;
+    if (group) {
+        const size_t ro = group->first * A.run_stride;
+        for (cplx<T> **f : {&A.z0, &A.z1, &A.zl0, &A.zl1, &A.u})
+            if (*f) *f += ro;
+        A.rw += group->first;
+        A.nu = group->nu, A.dt = group->dt;
+    }
+    const int    runs = group ? group->count : L->fft_runs;
     const int    nf   = OP == kXNs ? 5 : OP == kXZeta ? 0 : 3;
-    const double cols = (double)outer_count(g.ny, g.trn[1]) * g.trn[2] * L->fft_runs * sizeof(cplx<T>);
+    const double cols = (double)outer_count(g.ny, g.trn[1]) * g.trn[2] * runs * sizeof(cplx<T>);
     const double box  = box_bytes<T>(L, OP == kXSole ? (zeta_too ? 2 : 0) : OP == kXZeta ? 2 : A.zl0 ? 8 : 4);
     cudaEvent_t  pa   = prof_mark(L);
-    const cudaError_t e = x_fused<T, OP, INV>(plan_of<T>(L), A, L->fft_runs, L->nslots - slot, L->st);
+    const cudaError_t e = x_fused<T, OP, INV>(plan_of<T>(L), A, runs, L->nslots - slot, L->st);
     if (e == cudaErrorNotSupported) return SPM_OK;
     SPM_CUDA_CHECK(e);
     prof_done(L, pa, OP == kXZeta ? "x_zeta_u" : OP == kXNs ? "x_ns_update" : OP == kXProj ? "x_project" : "x_solenoidal",
@@ -842,11 +869,11 @@ int zeta_to_velocity(spm_ctx *L, int truncate, bool have_ux = false) {
     return z_pass<T>(L, U0, 3, false, L->g.trn[2]);
 }
 
-// NS_solver_slavedEuler (fluid_solver.cxx:348-374).  with_u: followed by
-// FIX_CELLxyz on `nr` runs and the velocity of the new zeta up to its inverse
-// X pass (zeta_to_velocity's have_ux).
+// NS_solver_slavedEuler (fluid_solver.cxx:348-374) of runs R[0..nr), each with
+// its own viscosity and time step.  with_u: followed by FIX_CELLxyz and the
+// velocity of the new zeta up to its inverse X pass (zeta_to_velocity's have_ux).
 template <typename T>
-int ns_solver(spm_ctx *L, int nr = 1, bool with_u = false) {
+int ns_solver(spm_ctx *L, spm_ctx *const *R, int nr, bool with_u = false) {
     // zeta -> u_hat (truncated) -> inverse x, y passes
     SPM_TRY(zeta_to_ux<T>(L));
     SPM_TRY((fft_strided_pass<T, +1>(L, U0, 3, 1, prune_inverse(L->g, 1))));
@@ -860,21 +887,32 @@ int ns_solver(spm_ctx *L, int nr = 1, bool with_u = false) {
     }
     L->launches++;
     SPM_TRY((fft_strided_pass<T, -1>(L, U0, 5, 1, prune_forward(L->g, 1))));
-    bool done;
-    if (with_u)
-        SPM_TRY((x_fused_pass<T, kXNs, true>(L, U0, 0, done)));
-    else
-        SPM_TRY((x_fused_pass<T, kXNs, false>(L, U0, 0, done)));
+    const std::vector<RunGroup> groups = run_groups(R, nr);
+    bool                        done   = false;
+    for (const RunGroup &gr : groups) {
+        if (with_u)
+            SPM_TRY((x_fused_pass<T, kXNs, true>(L, U0, 0, done, false, &gr)));
+        else
+            SPM_TRY((x_fused_pass<T, kXNs, false>(L, U0, 0, done, false, &gr)));
+        // whether it applies depends on the grid and the device alone
+        if (!done && gr.first > 0) return fail(SPM_ERR_CUDA, "fused X pass refused for part of a pool");
+        if (!done) break;
+    }
     if (done) return SPM_OK;
     SPM_TRY((fft_strided_pass<T, -1>(L, U0, 5, 0, prune_forward(L->g, 0))));
     // FP64: the update writes u_hat of the new zeta as well, one k_zeta_to_u
     // fewer.  Measured on B200 at 256^3 the fused update took 82 us against 60 +
     // 37 us; in FP32 it took 73 us against 44 + 25 us, so FP32 keeps two kernels.
     const bool u_too = with_u && L->fp64();
-    PLAUNCH(L, "k_ns_update", box_bytes<T>(L, (L->compensated() ? 13 : 9) + (u_too ? 3 : 0)), (k_ns_update<T, 2>),
-            L->box_grid(), 256, 0, L->g, L->cx<T>(Z0), L->cx<T>(Z1), L->cx<T>(U0), L->cx<T>(U1), L->cx<T>(U2),
-            L->cx<T>(A0), L->cx<T>(A1), L->ph.nu, L->ph.dt, L->fstride_c, L->zl<T>(0), L->zl<T>(1),
-            u_too ? L->rw : (const RunWords *)nullptr);
+    for (const RunGroup &gr : groups) {
+        const size_t ro = gr.first * L->fstride_c;
+        auto         at = [&](int slot) { return L->cx<T>(slot) + ro; };
+        cplx<T>     *l0 = L->zl<T>(0), *l1 = L->zl<T>(1);
+        PLAUNCH(L, "k_ns_update", box_bytes<T>(L, (L->compensated() ? 13 : 9) + (u_too ? 3 : 0)), (k_ns_update<T, 2>),
+                dim3(L->box_grid().x, gr.count), 256, 0, L->g, at(Z0), at(Z1), at(U0), at(U1), at(U2), at(A0), at(A1),
+                gr.nu, gr.dt, L->fstride_c, l0 ? l0 + ro : l0, l1 ? l1 + ro : l1,
+                u_too ? L->rw + gr.first : (const RunWords *)nullptr);
+    }
     if (!with_u) return SPM_OK;
     LAUNCH(L, k_fix_cell, (nr + 127) / 128, 128, 0, L->rw, nr);
     return u_too ? fft_strided_pass<T, +1>(L, U0, 3, 0, prune_inverse(L->g, 0)) : zeta_to_ux<T>(L);
@@ -1205,12 +1243,12 @@ int step_ns_runs(spm_ctx *L, spm_ctx *const *R, int nr) {
     }
     if (L->overlap) SPM_CUDA_CHECK(cudaEventRecord(L->ev_join, side));
     if (L->P.equation == SPM_EQ_SHEAR_NAVIER_STOKES) {  // lone runs only
-        SPM_TRY(ns_solver<T>(L));
+        SPM_TRY(ns_solver<T>(L, R, nr));
         SPM_TRY(shear_sustain<T>(L));
         LAUNCH(L, k_fix_cell, (nr + 127) / 128, 128, 0, L->rw, nr);
         SPM_TRY(zeta_to_velocity<T>(L, 1));
     } else {
-        SPM_TRY(ns_solver<T>(L, nr, true));
+        SPM_TRY(ns_solver<T>(L, R, nr, true));
         SPM_TRY(zeta_to_velocity<T>(L, 1, true));
     }
     if (L->overlap) SPM_CUDA_CHECK(cudaStreamWaitEvent(L->st, L->ev_join, 0));  // join
