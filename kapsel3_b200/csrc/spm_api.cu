@@ -216,6 +216,14 @@ int slots_for(const spm_params &p) {
     return p.precision == SPM_PREC_FP32_MIXED ? NSLOT + 2 : NSLOT;
 }
 
+// Lone spheres with the thermostat: the step's normals are drawn beside the fluid
+// solve into a buffer of six per particle (PRun::kick).
+bool draws_ahead(const spm_params &p) {
+    return (p.equation == SPM_EQ_NAVIER_STOKES || p.equation == SPM_EQ_SHEAR_NAVIER_STOKES) && p.kbt > 0.0 &&
+           p.n_particles > 0 && !p.rigid && p.janus_propulsion != SPM_JANUS_SQUIRMER &&
+           p.janus_propulsion != SPM_JANUS_OBSTACLE;
+}
+
 struct spm_pool;
 struct AvsOut;
 struct UdfOut;
@@ -1699,7 +1707,7 @@ int create_ctx(const spm_params &p, cudaStream_t stream, int pool_cap, spm_ctx *
         dev_alloc((void **)&c->mt, 625 * sizeof(unsigned int)) != cudaSuccess ||
         (lj_cell_list_applies(c->ph) &&
          dev_alloc((void **)&c->lj_list, ((size_t)lj_ncell(c->ph) * (1 + kLjBin) + np) * sizeof(int)) != cudaSuccess) ||
-        (!lead && p.kbt > 0.0 && p.n_particles > 0 &&
+        (!lead && draws_ahead(p) &&
          dev_alloc((void **)&c->noise, (size_t)np * 6 * sizeof(double)) != cudaSuccess)) {
         destroy_ctx(c);
         return fail(SPM_ERR_NOMEM, "small device buffers");
@@ -1838,7 +1846,8 @@ int spm_device_bytes(const spm_params *p, size_t *bytes) {
     const size_t nslot = (size_t)slots_for(*p);
     const bool   ns = p->equation == SPM_EQ_NAVIER_STOKES || p->equation == SPM_EQ_SHEAR_NAVIER_STOKES;
     const size_t sc = ns ? (size_t)p->n_particles * sekibun(*p).size() * 12 : 0;
-    *bytes = nslot * fld + (size_t)std::max(p->n_particles, 1) * kPWords * 8 + sc + 64 * 1024;
+    const size_t noise = draws_ahead(*p) ? (size_t)p->n_particles * 6 * 8 : 0;
+    *bytes = nslot * fld + (size_t)std::max(p->n_particles, 1) * kPWords * 8 + sc + noise + 64 * 1024;
     return SPM_OK;
 }
 

@@ -34,6 +34,31 @@ def test_params_default_and_bytes():
     assert b"NPX" in L.spm_last_error()
 
 
+def test_device_bytes_count_the_normals_and_descriptors():
+    """The thermostat's six normals per particle of a lone run; a pool's
+    descriptor of each run beside its fields and words."""
+    L, p, nb, arena, run = N.lib(), N.SpmParams(), C.c_size_t(), C.c_size_t(), C.c_size_t()
+    L.spm_params_default(C.byref(p))
+    p.n_particles = 100
+
+    def lone(kbt, janus=0):
+        p.kbt, p.janus_propulsion, p.janus_axis = kbt, janus, 3
+        assert L.spm_device_bytes(C.byref(p), C.byref(nb)) == 0
+        return nb.value
+
+    assert lone(1e-4) - lone(0.0) == 100 * 6 * 8
+    assert lone(1e-4, N.SPM_JANUS_OBSTACLE) == lone(0.0, N.SPM_JANUS_OBSTACLE)
+    p.janus_propulsion = 0
+
+    def pool(cap):
+        assert L.spm_pool_device_bytes(C.byref(p), cap, C.byref(arena), C.byref(run)) == 0
+        return arena.value
+
+    words = 4 * 8 + 4 * 4
+    fields = 11 * 32 * 32 * 17 * 16
+    assert pool(3) - pool(2) > fields + words + 100  # Phys alone is larger than that
+
+
 def test_udf_key_file_roundtrip():
     cfg = SPMConfig(npx=5, npy=6, npz=4, n_particles=3, a=3.0, a_xi=2.0, dt=0.04, kbt=1e-4,
                     fix_cell=(True, False, True), rotation=False, mass_ratio=1.0)
