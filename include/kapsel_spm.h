@@ -395,12 +395,17 @@ int spm_kernel_launches(spm_ctx *ctx, long long *count, int reset);
 
 /* ---- serving pool (no reference counterpart) ----------------------------
  * A pool holds independent Navier_Stokes runs of one grid size, DX and
- * precision.  Their fields share one slot-major device arena, and the runs'
- * particle buffers are listed in a device array, so every kernel of a pool
- * step is one launch over all runs.  The pool step can be replayed from a CUDA graph captured once per membership.  A run of
- * a pool is an spm_ctx: the whole-run getters above work on it (between
- * steps); spm_destroy refuses it (use spm_pool_release).  Releasing a run
- * moves the pool's last run into its slot; run handles stay valid. */
+ * precision; everything else may differ between them.  Their fields share one
+ * slot-major device arena, and the runs' particle buffers are listed in a
+ * device array, so a kernel of a pool step is one launch over all runs, except:
+ * the fluid's update is one per group of consecutive runs with the same
+ * viscosity and dt, the body forces of grids with an axis below 16 points
+ * (where no Lennard-Jones cell list applies) one per run, and the direct-load
+ * transform passes (SPM_NO_TMA=1) one per field slot.  The pool step can be replayed from a
+ * CUDA graph captured once per membership.  A run of a pool is an spm_ctx: the
+ * whole-run getters above work on it (between steps); spm_destroy refuses it
+ * (use spm_pool_release).  Releasing a run moves the pool's last run into its
+ * slot; run handles stay valid. */
 /* Device bytes of a pool arena of `capacity` runs of this grid, and of the
  * per-run particle buffers for grid->n_particles particles. */
 int spm_pool_device_bytes(const spm_params *grid, int capacity, size_t *arena_bytes, size_t *run_bytes);

@@ -1102,18 +1102,16 @@ int rigidity_projection(spm_ctx *L, int nr, int ts_inc) {
 
 int particle_blocks(spm_ctx *c) { return (c->ph.np + 127) / 128; }
 
-// The particle kernels' view of run c (PRun).
+// The particle kernels' view of run c (PRun), without its fields: what the
+// Lennard-Jones kernels need, whatever the fields' type.
 template <typename T>
-PRun<T> prun_of(spm_ctx *c) {
+PRun<T> prun_particles(spm_ctx *c) {
     PRun<T> R{};
     R.ph = c->ph, R.ps = c->ps;
     R.cells = c->cells, R.ncells = c->ncells;
     R.vel   = !c->rigid() && c->ph.janus_prop != SPM_JANUS_SQUIRMER;
     // obstacles draw no noise (fluct.cxx:23)
-    R.noise   = c->P.kbt > 0.0 && c->ph.janus_prop != SPM_JANUS_OBSTACLE;
-    R.phi_sum = c->real<T>(PHIS);
-    R.u0 = c->real<T>(U0), R.u1 = c->real<T>(U1), R.u2 = c->real<T>(U2);
-    R.f0 = c->real<T>(UP0), R.f1 = c->real<T>(UP1), R.f2 = c->real<T>(UP2);
+    R.noise = c->P.kbt > 0.0 && c->ph.janus_prop != SPM_JANUS_OBSTACLE;
     R.sc_idx = c->sc_idx, R.sc_w = c->sc_w;
     if (c->lj_list && lj_cell_list_applies(c->ph)) {
         R.lj_ncell   = lj_ncell(c->ph);
@@ -1124,6 +1122,14 @@ PRun<T> prun_of(spm_ctx *c) {
     if (c->rigid()) R.rid = c->rg.rid, R.f_lo = c->rg.f_lo;
     R.kick = R.vel && R.noise ? c->noise : nullptr;
     R.ts = c->ts_dev, R.mt = c->mt, R.err = c->err;
+    return R;
+}
+template <typename T>
+PRun<T> prun_of(spm_ctx *c) {
+    PRun<T> R = prun_particles<T>(c);
+    R.phi_sum = c->real<T>(PHIS);
+    R.u0 = c->real<T>(U0), R.u1 = c->real<T>(U1), R.u2 = c->real<T>(U2);
+    R.f0 = c->real<T>(UP0), R.f1 = c->real<T>(UP1), R.f2 = c->real<T>(UP2);
     return R;
 }
 
@@ -1139,7 +1145,7 @@ int lj_forces(spm_ctx *c, const Phys &ph, bool clear = true) {
                 c->rigid() ? c->rg.rid : nullptr, c->rigid() ? c->rg.f_lo : nullptr, (const double *)nullptr);
         return SPM_OK;
     }
-    PRun<double> R = prun_of<double>(c);
+    PRun<double> R = prun_particles<double>(c);
     R.ph           = ph;
     if (ph.lj_on && ph.janus_prop != 3) {
         if (clear) SPM_CUDA_CHECK(cudaMemsetAsync(R.lj_count, 0, (size_t)R.lj_ncell * sizeof(int), c->st));
