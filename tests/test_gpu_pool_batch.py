@@ -47,3 +47,23 @@ def test_pool_runs_match_lone_runs(gpu, order, use_graph):
             for k in ("x", "v", "omega", "q", "f_hydro_previous", "fr_previous"):
                 assert rel(got[k], p[k]) <= 1e-12, (c.n_particles, k)
             assert rel(pool.velocity(r, c.shape), u) <= 1e-12, c.n_particles
+
+
+@pytest.mark.parametrize("shape", [(3, 5, 5), (5, 5, 3)])
+def test_pool_without_a_cell_list(gpu, shape):
+    """An axis of 8 points (no Lennard-Jones forces there): the body forces, one launch per run."""
+    cfgs = [SPMConfig(npx=shape[0], npy=shape[1], npz=shape[2], n_particles=n, a=1.0, a_xi=1.0, dt=0.05,
+                      lj_truncate="NONE", body_force=(1e-3, 0.0, 0.0)) for n in (0, 9, 2)]
+    parts = [make_particles(c, seed=50 + i, v_sd=1e-3) for i, c in enumerate(cfgs)]
+    with Pool(cfgs[0], precision=N.SPM_PREC_FP64, capacity=3) as pool:
+        runs = [pool.admit(c, p) for c, p in zip(cfgs, parts)]
+        pool.step(3)
+        pool.synchronize()
+        got = [unpack_particles(pool.particles(r, c.n_particles)) for r, c in zip(runs, cfgs)]
+    for c, p, g in zip(cfgs, parts, got):
+        with SPMRun(c) as run:
+            run.initialize(p)
+            run.step(3)
+            want = run.particles()
+        for k in ("x", "v", "f_hydro_previous", "fr_previous"):
+            assert rel(g[k], want[k]) <= 1e-12, (c.n_particles, k)

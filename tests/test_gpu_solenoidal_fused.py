@@ -10,6 +10,7 @@ import pytest
 from kapsel3_b200 import _native as N
 from kapsel3_b200.spm import SPMRun
 from kapsel3_b200.udf import EQ_EL, SPMConfig, make_particles
+from kernel_names import step_kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -19,7 +20,10 @@ def _run(cfg, parts, no_tma, monkeypatch, prec):
     with SPMRun(cfg, precision=prec) as run:
         run.initialize(parts)
         run.step(3)
-        return run.particles(), run.velocity()
+        out = run.particles(), run.velocity()
+        fused = not no_tma and cfg.shape[0] <= (256 if prec == N.SPM_PREC_FP64 else 512)
+        assert ("x_solenoidal" in step_kernels(run)) == fused
+        return out
 
 
 def _close(cfg, monkeypatch, prec, tol):

@@ -8,6 +8,7 @@ import pytest
 from kapsel3_b200 import _native as N
 from kapsel3_b200.spm import SPMRun
 from kapsel3_b200.udf import SPMConfig, make_particles
+from kernel_names import step_kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -17,6 +18,8 @@ def test_fused_wait_runs_out(gpu, prec):
     cfg = SPMConfig(npx=5, npy=5, npz=5, n_particles=2, a=4.0, a_xi=2.0, dt=0.05)
     parts = make_particles(cfg, seed=7, v_sd=1e-3, random_orientation=True)
     with SPMRun(cfg, precision=prec) as run:
+        run.initialize(parts)
+        assert "x_ns_update" in step_kernels(run)  # the third pass is the fused one
         run.initialize(parts)
         run.step(3)
         want = run.particles()
