@@ -205,6 +205,11 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
     constexpr int      ND         = NF > 0 ? NF : 1;  // divisor of the load sequence
     constexpr int      S          = OP == kXZeta ? 1 : kXRing;
     constexpr unsigned tile_bytes = (unsigned)(N * W * sizeof(cplx<T>));
+    // two CTAs of 256 threads leave a thread 128 registers (FP32 at 256 points): the
+    // values that the branch-free loads of zeta keep alive then spill (112 bytes in
+    // kXNs, none with a predicate per mode; ten steps 10132 -> 10008 us).  With 255
+    // registers the branch-free form is faster (512 points FP32: 7731 against 7597 us)
+    constexpr bool kFewRegs = N >= 256 && W * N1 >= 256;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     cplx<T> *buf = reinterpret_cast<cplx<T> *>(smem_raw);
     double  *skx = reinterpret_cast<double *>(buf + (size_t)S * N * W);  // kx of index n
@@ -383,8 +388,9 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
             }
         }
         // k-space stage: a0, a1 become zeta.  zeta of kXChunk modes at a time is
-        // loaded without branches (XModes::zeta_index), so its loads are in flight
-        // together; what a mode outside the box loads is dropped.
+        // loaded without branches (XModes::zeta_index; kFewRegs: its own modes only),
+        // so its loads are in flight together; what a mode outside the box loads is
+        // dropped.
         // e^{x + y} - 1 = ex + ey + ex ey for x, y <= 0 has no cancellation, so a
         // mode costs no exponential of its own.
         const double dkyz2 = dky * dky + dkz * dkz;
@@ -397,9 +403,11 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
             for (int j = 0; j < kXChunk; j++) {
                 const int m = mc + j;
                 if (m >= N2 || !M::maybe(m)) continue;
-                const unsigned idx = (unsigned)M::zeta_index(g, m) * nst + line;
-                z0[j] = pz0[idx], z1[j] = pz1[idx];
-                if (OP != kXZeta && comp) l0[j] = pl0[idx], l1[j] = pl1[idx];
+                const unsigned idx = (unsigned)(kFewRegs ? g + N1 * m : M::zeta_index(g, m)) * nst + line;
+                const bool     ld  = !kFewRegs || keep(m);
+                if (kFewRegs) z0[j] = z1[j] = l0[j] = l1[j] = cplx<T>{0, 0};
+                if (ld) z0[j] = pz0[idx], z1[j] = pz1[idx];
+                if (OP != kXZeta && comp && ld) l0[j] = pl0[idx], l1[j] = pl1[idx];
             }
 #pragma unroll
             for (int j = 0; j < kXChunk; j++) {
