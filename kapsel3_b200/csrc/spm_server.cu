@@ -366,8 +366,8 @@ void spm_server::loop() {
         }
         if (admit_some()) progressed = true;
         // Drop pools that stayed empty for pool_idle_s, or at once when a
-        // queued request is waiting: freeing an arena waits for the whole
-        // device, so a pool that empties and refills within a moment keeps it.
+        // queued request is waiting; one that empties and refills within a
+        // moment keeps its arena and plans.
         bool waiting = false;
         {
             std::lock_guard<std::mutex> lk(mu);

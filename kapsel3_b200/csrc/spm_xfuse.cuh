@@ -484,7 +484,8 @@ __global__ void __launch_bounds__(W *Split<N>::N1, N >= 256 ? 2 : 1)
                         }
                         const T kx = skt[g + N1 * m], ikx = sik[g + N1 * m];
                         // formed again for each component: kept, its 12 values per thread spill
-                        // (ten steps at 256^3: FP64 15674 against 15280 us, FP32 10143 against 9929)
+                        // (beyond the 64 to 80 bytes that FP64 spills as it is; ten steps at
+                        // 256^3: FP64 15674 against 15280 us, FP32 10143 against 9929)
                         const T ik2 = (T)x_reciprocal<T>(skx[g + N1 * m] * skx[g + N1 * m] + dkyz2);
                         if (m == 0)
                             v[m] = x_velocity<T, D.value, true>(kx, kyt, kzt, ik2, ikx, kx0, ky0, kz_ky, a0[m], a1[m]);
